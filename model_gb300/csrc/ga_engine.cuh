@@ -26,47 +26,6 @@ namespace ga {
 
 static inline int cdiv(long a, long b) { return (int)((a + b - 1) / b); }
 
-// Factor plan of the shared-memory FFT of length n.  order (autotuned):
-// 0 radix 4 first, then 2, then odd primes; 1 the radix 2 first; 2 radix 2
-// only; 3 odd primes first.  Returns nfac = 0 for an order that gives no new
-// plan for this n.
-static inline FftPlan make_fft_plan(int n, int order = 0)
-{
-    FftPlan P;
-    std::memset(&P, 0, sizeof(P));
-    P.n = n;
-    int m = n, c4 = 0, c2 = 0, odd[24], no = 0;
-    while (m % 4 == 0) { c4++; m /= 4; }
-    if (m % 2 == 0) { c2 = 1; m /= 2; }
-    for (int f = 3; m > 1 && no < 24;) {
-        if (m % f == 0) { odd[no++] = f; m /= f; }
-        else f += 2;
-    }
-    if (order == 1 && c2 == 0) return P;   // same as order 0
-    if (order == 2) {
-        if (c4 == 0) return P;
-        c2 += 2 * c4;
-        c4 = 0;
-    }
-    if (order == 3 && (no == 0 || (c4 == 0 && c2 == 0))) return P;
-    auto push = [&](int f) { if (P.nfac < 24) P.fac[P.nfac++] = f; };
-    if (order == 3)
-        for (int t = 0; t < no; t++) push(odd[t]);
-    if (order == 1)
-        for (int t = 0; t < c2; t++) push(2);
-    for (int t = 0; t < c4; t++) push(4);
-    if (order != 1)
-        for (int t = 0; t < c2; t++) push(2);
-    if (order != 3)
-        for (int t = 0; t < no; t++) push(odd[t]);
-    int ns = 1;
-    for (int f = 0; f < P.nfac; f++) {
-        P.nslog[f] = (ns & (ns - 1)) == 0 ? __builtin_ctz(ns) : -1;
-        ns *= P.fac[f];
-    }
-    return P;
-}
-
 template <typename T>
 struct Lin;
 
@@ -97,9 +56,9 @@ class Engine : public EngineBase {
     unsigned char *ppm_has = nullptr;
     T *ppm_topq = nullptr, *ppm_topm = nullptr, *ppm_cin = nullptr, *ppm_carry = nullptr;
     double *staging = nullptr;
-    int KTy = 1, KTx = 1, lgKTy = 0, lgKTx = 0, TC = 64;
+    int KTy = 1, KTx = 1, TC = 64;  // lines per y block (level pairs) and x block (levels); Thomas columns per block
     int psx = 0;  // point stride of the fused spectral-x kernel (0: unfused path)
-    int sx_threads = 256;  // threads of a fused spectral-x block (autotuned)
+    int sx_threads = 256;  // threads of a fused spectral-x block (set from the grid, autotuned)
     // FP32: the fused x kernel as clusters of two CTAs per y-wavenumber
     // (autotuned; GA_SPECTRAL_X=pair makes it the default)
     bool sx_pair = false;
@@ -174,6 +133,28 @@ class Engine : public EngineBase {
         cudaStreamWaitEvent(stream, ev_join, 0);
     }
     int hyd_L = 1;               // y-lines per block of its x transforms
+
+    void set_kty(int kt)
+    {
+        KTy = kt;
+        smem_y = fft_bytes(kp.nj, kt, sizeof(T2));
+    }
+    void set_ktx(int kt)
+    {
+        KTx = kt;
+        smem_x = fft_bytes(kp.ni, kt, sizeof(T2));
+    }
+    // block of the level-tiled transforms of n points: a row of threads per
+    // radix-8 butterfly, 128 to 256 threads
+    static dim3 fft_block(int n, int kt)
+    {
+        const int rows = std::min(std::max(cdiv(n, 8), std::max(1, 128 / kt)), std::max(1, 256 / kt));
+        return dim3(kt, rows);
+    }
+    dim3 block_y() const { return fft_block(kp.nj, KTy); }
+    dim3 block_x() const { return fft_block(kp.ni, KTx); }
+    dim3 grid_y() const { return dim3(cdiv(level_pairs(NZ), KTy), kp.ni); }
+    dim3 grid_x() const { return dim3(cdiv(NZ - 2, KTx), kp.nh); }
 
     // Fornberg's recurrence for finite-difference weights: c[i*(m+1)+d] is the
     // weight of point x[i] in derivative d at z (util.cpp:199-247)
@@ -314,7 +295,8 @@ class Engine : public EngineBase {
         d_err = dalloc<int>(2);  // [0] Kessler, [1] staging (kErrStaging)
         const int periodic = c->periodic_ew_boundaries;
         const int ni = periodic ? NX - 6 : NX, nj = NY;
-        spec = dalloc<T2>((size_t)ni * nj * NZ);
+        const int nh = spec_nh(nj), nzs = spec_nzs(NZ);
+        spec = dalloc<T2>((size_t)ni * nh * nzs);
         btab = dalloc<T>((size_t)BT_COUNT * NZ);
 
         // ---- scalars (initialize_globals, initializer.cpp:168-179) ----
@@ -322,6 +304,7 @@ class Engine : public EngineBase {
         std::memset(&kp, 0, sizeof(kp));
         kp.nx = NX; kp.ny = NY; kp.nz = NZ; kp.n = N;
         kp.ni = ni; kp.nj = nj; kp.ioff = periodic ? 3 : 0;
+        kp.nh = nh; kp.nzs = nzs;
         kp.periodic = periodic; kp.moist = moist; kp.rf = c->rain_fallout;
         kp.dtx = (T)(dt / dx); kp.dty = (T)(dt / dy); kp.dtz = (T)(dt / dz); kp.dt = (T)dt;
         kp.one_d_dx = (T)(1.0 / dx); kp.one_d_dy = (T)(1.0 / dy); kp.one_d_dz = (T)(1.0 / dz);
@@ -377,11 +360,11 @@ class Engine : public EngineBase {
         kp.nb = NY - jn; kp.ne = NY; kp.sb = 0; kp.se = js;
 
         // ---- pressure solver tables (init_fft3d, pressure.cpp:724-797) ----
-        std::vector<double> hcoef((size_t)ni * nj), kw(ni), lw(nj);
+        std::vector<double> hcoef((size_t)ni * nh), kw(ni), lw(nj);
         for (int i = 0; i < ni; i++) kw[i] = (double)i * 2 * trigpi / ((double)ni);
         for (int j = 0; j < nj; j++) lw[j] = (double)j * 2 * trigpi / ((double)nj);
         for (int i = 0; i < ni; i++)
-            for (int j = 0; j < nj; j++) hcoef[(size_t)i * nj + j] = cos(kw[i]) + cos(lw[j]) - 2.0;
+            for (int j = 0; j < nh; j++) hcoef[(size_t)i * nh + j] = cos(kw[i]) + cos(lw[j]) - 2.0;
         kp.hcoef = upload(hcoef);
         std::vector<double> ac(NZ, 0.0), cc(NZ, 0.0), vc(NZ, 0.0);
         const double dz2 = dz * dz;
@@ -527,20 +510,16 @@ class Engine : public EngineBase {
         };
         tw_i = twiddles(ni);
         tw_j = twiddles(nj);
-        // power-of-two level tiles for the y and x transforms (~32 KiB per buffer)
-        auto pow2_tile = [&](int n, int *lg) {
-            const long budget = 32 * 1024;
-            long want = std::max(1L, budget / (long)(2 * n * sizeof(T2)));
-            int kt = 1, l = 0;
-            while ((kt << 1) <= want && (kt << 1) <= 2 * (NZ - 2)) { kt <<= 1; l++; }
-            while (kt > 1 && (kt >> 1) >= NZ - 2) { kt >>= 1; l--; }
-            *lg = l;
+        // lines per block of the y (level pairs) and x (levels) transforms:
+        // eight 8-byte lines are 64-byte rows in x and 64-byte level runs in y,
+        // fewer where the two buffers of a long line would leave one block per SM
+        auto line_tile = [&](int n, int lines) {
+            int kt = 8;
+            while (kt > 1 && (fft_bytes(n, kt, sizeof(T2)) > 100 * 1024 || kt / 2 >= lines)) kt >>= 1;
             return kt;
         };
-        KTy = pow2_tile(nj, &lgKTy);
-        KTx = pow2_tile(ni, &lgKTx);
-        smem_y = 2 * (size_t)nj * KTy * sizeof(T2);
-        smem_x = 2 * (size_t)ni * KTx * sizeof(T2);
+        set_kty(line_tile(nj, level_pairs(NZ)));
+        set_ktx(line_tile(ni, NZ - 2));
         smem_th = (size_t)TC * (NZ | 1) * (sizeof(T2) + sizeof(T));
         const int optin = 200 * 1024;
         {   // fused x transform + Thomas when all levels of a wavenumber fit.  The
@@ -552,6 +531,10 @@ class Engine : public EngineBase {
             if (2 * (size_t)ni * ps * sizeof(T2) <= (size_t)optin) psx = ps;
             else if (2 * (size_t)ni * (nl | 1) * sizeof(T2) <= (size_t)optin) psx = nl | 1;
             smem_sx = 2 * (size_t)ni * psx * sizeof(T2);
+            // one radix-8 butterfly per thread: the block's passes are chains
+            // of shared-memory round trips, so idle or looping threads cost time
+            const int bx = std::min(nl, 64);
+            sx_threads = std::min(std::max(bx * cdiv(ni, 8), 256), sizeof(T) == 4 ? 1024 : 512);
         }
         cudaFuncSetAttribute(k_spectral_x<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
         cudaFuncSetAttribute(k_spectral_x_1k<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
@@ -1118,11 +1101,9 @@ class Engine : public EngineBase {
     {
         KFields<T> F = fields();
         const T sdt = (T)(step * cfg.dt);
-        const int nkt_y = cdiv(NZ - 2, KTy), nkt_x = cdiv(NZ - 2, KTx);
-        const dim3 by_y(KTy, std::max(1, 256 / KTy)), by_x(KTx, std::max(1, 256 / KTx));
         {
             ProfScope ps(this, PC_DIV_FFT_Y, 1);
-            k_div_fft_y<T><<<dim3(nkt_y, kp.ni), by_y, smem_y, stream>>>(kp, F, spec, plan_j, tw_j, sdt, KTy);
+            k_div_fft_y<T><<<grid_y(), block_y(), smem_y, stream>>>(kp, F, spec, plan_j, tw_j, sdt, KTy);
         }
         if (mid_solve) {  // work queued beside the rest of the solve (the x solve leaves SMs idle)
             auto fn = std::move(mid_solve);
@@ -1137,35 +1118,35 @@ class Engine : public EngineBase {
             if (pair) {
                 if constexpr (sizeof(T) == 4) {
                     const int bh = std::min((nl + 1) / 2, 32);
-                    k_spectral_x_pair<T><<<2 * kp.nj, dim3(bh, std::max(1, sx_threads / bh)), smem_sxp, stream>>>(
+                    k_spectral_x_pair<T><<<2 * kp.nh, dim3(bh, std::max(1, sx_threads / bh)), smem_sxp, stream>>>(
                         kp, spec, plan_i, tw_i, sx_pair_layout(NZ));
                 }
             } else if (sx_threads > 512) {
-                k_spectral_x_1k<T><<<kp.nj, dim3(bx, sx_threads / bx), smem_sx, stream>>>(kp, spec, plan_i, tw_i, psx);
+                k_spectral_x_1k<T><<<kp.nh, dim3(bx, sx_threads / bx), smem_sx, stream>>>(kp, spec, plan_i, tw_i, psx);
             } else {
-                k_spectral_x<T><<<kp.nj, dim3(bx, std::max(1, sx_threads / bx)), smem_sx, stream>>>(kp, spec, plan_i,
+                k_spectral_x<T><<<kp.nh, dim3(bx, std::max(1, sx_threads / bx)), smem_sx, stream>>>(kp, spec, plan_i,
                                                                                                    tw_i, psx);
             }
             launches += 1;
         } else {
             {
                 ProfScope ps(this, PC_FFT_X, 1);
-                k_fft_x<T><<<dim3(nkt_x, kp.nj), by_x, smem_x, stream>>>(kp, spec, plan_i, tw_i, 0, KTx);
+                k_fft_x<T><<<grid_x(), block_x(), smem_x, stream>>>(kp, spec, plan_i, tw_i, 0, KTx);
             }
-            const long ncol = (long)kp.ni * kp.nj;
+            const long ncol = (long)kp.ni * kp.nh;
             {
                 ProfScope ps(this, PC_THOMAS, 1);
                 k_thomas<T><<<cdiv(ncol, TC), 256, smem_th, stream>>>(kp, spec, TC);  // 256 threads stage, TC solve
             }
             {
                 ProfScope ps(this, PC_FFT_X, 1);
-                k_fft_x<T><<<dim3(nkt_x, kp.nj), by_x, smem_x, stream>>>(kp, spec, plan_i, tw_i, 1, KTx);
+                k_fft_x<T><<<grid_x(), block_x(), smem_x, stream>>>(kp, spec, plan_i, tw_i, 1, KTx);
             }
             launches += 3;
         }
         {
             ProfScope ps(this, PC_IFFT_Y_PI, 1);
-            k_ifft_y_pi<T><<<dim3(nkt_y, kp.ni), by_y, smem_y, stream>>>(kp, F, spec, plan_j, tw_j, KTy);
+            k_ifft_y_pi<T><<<grid_y(), block_y(), smem_y, stream>>>(kp, F, spec, plan_j, tw_j, KTy);
         }
         launches += 2;
     }
@@ -1809,17 +1790,11 @@ class Engine : public EngineBase {
             info += line;
         }
         // y transforms: level tile, then factor order
-        auto set_kty = [&](int kt) {
-            KTy = kt;
-            lgKTy = 0;
-            while ((1 << lgKTy) < kt) lgKTy++;
-            smem_y = 2 * (size_t)kp.nj * KTy * sizeof(T2);
-        };
         {
             float best = 1e30f;
             int bk = KTy;
-            for (int kt = 1; kt <= 64 && kt <= 2 * (NZ - 2); kt <<= 1) {
-                if (2 * (size_t)kp.nj * kt * sizeof(T2) > 200 * 1024) break;
+            for (int kt = 1; kt <= 64 && kt < 2 * level_pairs(NZ); kt <<= 1) {
+                if (fft_bytes(kp.nj, kt, sizeof(T2)) > 200 * 1024) break;
                 set_kty(kt);
                 const float t = timeit([&] { solve_pressure(1. / 3.); });
                 if (t < best) { best = t; bk = kt; }
@@ -1838,7 +1813,7 @@ class Engine : public EngineBase {
             }
             plan_order_j = bo;
             plan_j = make_fft_plan(kp.nj, bo);
-            std::snprintf(line, sizeof line, "y level tile %d, y FFT order %d; ", bk, bo);
+            std::snprintf(line, sizeof line, "y level tile %d pairs, y FFT order %d; ", bk, bo);
             info += line;
             // x transforms: factor order (and the level tile of the unfused path)
             float bx = bestp;
@@ -1860,7 +1835,8 @@ class Engine : public EngineBase {
                 int bt = keep;
                 bool bp = false;
                 sx_pair = false;
-                for (int nt : {512, 1024}) {
+                for (int nt : {256, 512, 1024}) {
+                    if (nt == keep) continue;
                     sx_threads = nt;
                     const float t = timeit([&] { solve_pressure(1. / 3.); });
                     if (t < bx) { bx = t; bt = nt; }
@@ -1884,21 +1860,13 @@ class Engine : public EngineBase {
                 psx = 0;
                 int bkx = -1;
                 for (int kt = 1; kt <= 64 && kt <= 2 * (NZ - 2); kt <<= 1) {
-                    if (2 * (size_t)kp.ni * kt * sizeof(T2) > 200 * 1024) break;
-                    KTx = kt;
-                    smem_x = 2 * (size_t)kp.ni * KTx * sizeof(T2);
+                    if (fft_bytes(kp.ni, kt, sizeof(T2)) > 200 * 1024) break;
+                    set_ktx(kt);
                     const float t = timeit([&] { solve_pressure(1. / 3.); });
                     if (t < bx || (keep_psx == 0 && bkx < 0)) { bx = std::min(bx, t); bkx = kt; }
                 }
-                if (bkx > 0) {
-                    KTx = bkx;
-                } else {
-                    psx = keep_psx;
-                    KTx = keep_kt;
-                }
-                lgKTx = 0;
-                while ((1 << lgKTx) < KTx) lgKTx++;
-                smem_x = 2 * (size_t)kp.ni * KTx * sizeof(T2);
+                set_ktx(bkx > 0 ? bkx : keep_kt);
+                if (bkx <= 0) psx = keep_psx;
                 if (psx == 0) std::snprintf(line, sizeof line, "x level tile %d, ", KTx);
                 else std::snprintf(line, sizeof line, "x fused%s, %d threads, ", sx_pair ? " (CTA pairs)" : "",
                                    sx_threads);

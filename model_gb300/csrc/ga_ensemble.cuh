@@ -109,7 +109,7 @@ __global__ void kb_div_fft_y(const KParams<T> *P, const KFields<T> *F, const Mem
         const KParams<T> &p = P[m];
         const MemberAux<T> &a = A[m];
         const long lb = vb - pre[m];
-        const long nkt = (p.nz - 2 + a.KTy - 1) / a.KTy;  // level tiles of a plane run next to each other
+        const long nkt = (level_pairs(p.nz) + a.KTy - 1) / a.KTy;  // level tiles of a plane run next to each other
         div_fft_y_body(p, F[m], a.spec, a.plan_j, a.tw_j, (T)(step * p.dt_d), a.KTy, (int)(lb / nkt),
                        (int)(lb % nkt));
         __syncthreads();
@@ -165,7 +165,7 @@ __global__ void kb_ifft_y_pi(const KParams<T> *P, const KFields<T> *F, const Mem
         const KParams<T> &p = P[m];
         const MemberAux<T> &a = A[m];
         const long lb = vb - pre[m];
-        const long nkt = (p.nz - 2 + a.KTy - 1) / a.KTy;
+        const long nkt = (level_pairs(p.nz) + a.KTy - 1) / a.KTy;
         ifft_y_pi_body(p, F[m], a.spec, a.plan_j, a.tw_j, a.KTy, (int)(lb / nkt), (int)(lb % nkt));
         __syncthreads();
     }
@@ -396,7 +396,7 @@ class Ensemble : public EnsembleBase {
     bool ktx_fits(int kt) const
     {
         for (auto *e : mem)
-            if (kt > 2 * (e->NZ - 2) || 2 * (size_t)e->kp.ni * kt * sizeof(typename V2<T>::t) > 200 * 1024)
+            if (kt > 2 * (e->NZ - 2) || fft_bytes(e->kp.ni, kt, sizeof(typename V2<T>::t)) > 200 * 1024)
                 return false;
         return true;
     }
@@ -427,11 +427,11 @@ class Ensemble : public EnsembleBase {
                 case EK_MIRROR: c = cdiv(2L * (e.NX + e.NY - 2) * (e.NZ - 2), 256); break;
                 case EK_DIVY:
                 case EK_IFFTY:
-                    c = (long)e.kp.ni * cdiv(e.NZ - 2, e.KTy);
+                    c = (long)e.kp.ni * cdiv(level_pairs(e.NZ), e.KTy);
                     sm = std::max(sm, e.smem_y);
                     break;
                 case EK_SX:
-                    c = e.kp.nj;
+                    c = e.kp.nh;
                     sm = std::max(sm, e.smem_sx);
                     break;
                 case EK_POST:
@@ -439,11 +439,11 @@ class Ensemble : public EnsembleBase {
                     break;
                 case EK_KES: c = cdiv((long)(e.NX - 2) * (e.NY - 2) * (e.NZ - 2), 128); break;
                 case EK_FX:
-                    c = (long)e.kp.nj * cdiv(e.NZ - 2, KTx);
-                    sm = std::max(sm, 2 * (size_t)e.kp.ni * KTx * sizeof(typename V2<T>::t));
+                    c = (long)e.kp.nh * cdiv(e.NZ - 2, KTx);
+                    sm = std::max(sm, fft_bytes(e.kp.ni, KTx, sizeof(typename V2<T>::t)));
                     break;
                 case EK_TH:
-                    c = cdiv((long)e.kp.ni * e.kp.nj, TC);
+                    c = cdiv((long)e.kp.ni * e.kp.nh, TC);
                     sm = std::max(sm, (size_t)TC * (e.NZ | 1) * (sizeof(typename V2<T>::t) + sizeof(T)));
                     break;
                 }
@@ -566,10 +566,7 @@ class Ensemble : public EnsembleBase {
             std::vector<int> keep(nmem);
             for (int m = 0; m < nmem; m++) keep[m] = mem[m]->KTy;
             auto set_kty = [&](int kt) {
-                for (auto *e : mem) {
-                    e->KTy = kt;
-                    e->smem_y = 2 * (size_t)e->kp.nj * kt * sizeof(T2);
-                }
+                for (auto *e : mem) e->set_kty(kt);
                 tables_dirty = true;
                 refresh_tables();
                 build_prefixes();
@@ -577,10 +574,10 @@ class Ensemble : public EnsembleBase {
             auto chain = [&] {
                 const KFields<T> *G = d_f[rot];
                 kb_mirror<T><<<grid[EK_MIRROR], 256, 0, stream>>>(d_p, G, d_pre[EK_MIRROR], nmem);
-                kb_div_fft_y<T><<<grid[EK_DIVY], dim3(16, 16), smem[EK_DIVY], stream>>>(d_p, G, d_aux,
+                kb_div_fft_y<T><<<grid[EK_DIVY], dim3(8, 32), smem[EK_DIVY], stream>>>(d_p, G, d_aux,
                                                                                        d_pre[EK_DIVY], nmem, 1. / 3.);
                 launch_sx();
-                kb_ifft_y_pi<T><<<grid[EK_IFFTY], dim3(16, 16), smem[EK_IFFTY], stream>>>(d_p, G, d_aux,
+                kb_ifft_y_pi<T><<<grid[EK_IFFTY], dim3(8, 32), smem[EK_IFFTY], stream>>>(d_p, G, d_aux,
                                                                                          d_pre[EK_IFFTY], nmem);
             };
             float best = 1e30f;
@@ -588,7 +585,7 @@ class Ensemble : public EnsembleBase {
             for (int kt = 1; kt <= 64; kt <<= 1) {
                 bool fits = true;
                 for (auto *e : mem)
-                    fits = fits && kt <= 2 * (e->NZ - 2) && 2 * (size_t)e->kp.nj * kt * sizeof(T2) <= 200 * 1024;
+                    fits = fits && kt < 2 * level_pairs(e->NZ) && fft_bytes(e->kp.nj, kt, sizeof(T2)) <= 200 * 1024;
                 if (!fits) break;
                 set_kty(kt);
                 const float t = timeit(chain);
@@ -597,10 +594,7 @@ class Ensemble : public EnsembleBase {
             if (bk > 0) {
                 set_kty(bk);
             } else {
-                for (int m = 0; m < nmem; m++) {
-                    mem[m]->KTy = keep[m];
-                    mem[m]->smem_y = 2 * (size_t)mem[m]->kp.nj * keep[m] * sizeof(T2);
-                }
+                for (int m = 0; m < nmem; m++) mem[m]->set_kty(keep[m]);
                 tables_dirty = true;
                 refresh_tables();
                 build_prefixes();
@@ -711,10 +705,10 @@ class Ensemble : public EnsembleBase {
             const int what = ADV_UV | ADV_WB | ADV_TH | (moist ? (ADV_Q | ADV_ZERO) : 0);
             launch_advect(F, st, what);
             kb_mirror<T><<<grid[EK_MIRROR], 256, 0, stream>>>(d_p, F, d_pre[EK_MIRROR], nmem);
-            kb_div_fft_y<T><<<grid[EK_DIVY], dim3(16, 16), smem[EK_DIVY], stream>>>(d_p, F, d_aux, d_pre[EK_DIVY],
+            kb_div_fft_y<T><<<grid[EK_DIVY], dim3(8, 32), smem[EK_DIVY], stream>>>(d_p, F, d_aux, d_pre[EK_DIVY],
                                                                                    nmem, st);
             launch_sx();
-            kb_ifft_y_pi<T><<<grid[EK_IFFTY], dim3(16, 16), smem[EK_IFFTY], stream>>>(d_p, F, d_aux, d_pre[EK_IFFTY],
+            kb_ifft_y_pi<T><<<grid[EK_IFFTY], dim3(8, 32), smem[EK_IFFTY], stream>>>(d_p, F, d_aux, d_pre[EK_IFFTY],
                                                                                      nmem);
             const int fu = PF_PROJECT | PF_SPONGE | PF_VBC, ft = PF_SPONGE | PF_VBC, fq = PF_ZERO | PF_SPONGE | PF_VBC;
             launch_post(F, make_int4(fu, fu, fu, ft), make_int4(fq, fq, fq, 0), st);

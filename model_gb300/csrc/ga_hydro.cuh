@@ -128,7 +128,7 @@ __global__ void k_hyd_fft(KParams<T> p, HydArgs<T> h, FftPlan P, const typename 
             a[i * L + l] = v;
         }
     __syncthreads();
-    T2 *r = fft_smem<T, T2>(a, b, L, P, tw, inv != 0, L);
+    const T2 *r = inv ? fft_smem<true, T, T2>(a, b, L, P, tw, L) : fft_smem<false, T, T2>(a, b, L, P, tw, L);
     const T n = (T)p.nx;
     for (int i = threadIdx.y; i < p.nx; i += blockDim.y)
         for (int l = threadIdx.x; l < lt; l += blockDim.x) {

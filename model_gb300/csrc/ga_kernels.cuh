@@ -30,6 +30,7 @@ struct KParams {
     long n;
     double dt_d;             // time step in double (step constants are formed from it)
     int ni, nj, ioff;        // spectral grid and its first physical column
+    int nh, nzs;             // stored y-wavenumbers (nj/2 + 1) and level stride of the spectral buffer
     int periodic, moist, rf;
     T dtx, dty, dtz, dt, one_d_dx, one_d_dy, one_d_dz;
     // vertical columns [nz] and Coriolis [ny]
@@ -993,6 +994,53 @@ struct FftPlan {
     int nslog[24];  // log2 of the sub-transform size before each pass, -1 if not a power of two
 };
 
+// Factor plan of the shared-memory FFT of length n.  order (autotuned):
+// 0 radix 8 first, then 4, 2 and the odd primes; 1 radix 4 instead of 8;
+// 2 the odd primes first; 3 the radix 4 or 2 before the 8s.  Returns nfac = 0
+// for an order that gives no new plan for this n.
+static inline FftPlan make_fft_plan(int n, int order = 0)
+{
+    FftPlan P;
+    std::memset(&P, 0, sizeof(P));
+    P.n = n;
+    int m = n, e2 = 0, odd[24], no = 0;
+    while (m % 2 == 0) { e2++; m /= 2; }
+    for (int f = 3; m > 1 && no < 24;) {
+        if (m % f == 0) { odd[no++] = f; m /= f; }
+        else f += 2;
+    }
+    // the fewest passes for 2^e2: 8s, with one or two 4s or a 2 for the rest
+    int c8 = e2 / 3, c4 = 0, c2 = 0;
+    if (e2 % 3 == 2) c4 = 1;
+    else if (e2 % 3 == 1 && c8 > 0) { c8--; c4 = 2; }
+    else if (e2 % 3 == 1) c2 = 1;
+    if (order == 1) {
+        if (c8 == 0) return P;
+        c8 = 0;
+        c4 = e2 / 2;
+        c2 = e2 % 2;
+    }
+    if (order == 2 && (no == 0 || e2 == 0)) return P;
+    if (order == 3 && (c8 == 0 || c4 + c2 == 0)) return P;
+    auto push = [&](int f, int times) {
+        for (int t = 0; t < times && P.nfac < 24; t++) P.fac[P.nfac++] = f;
+    };
+    if (order == 2)
+        for (int t = 0; t < no; t++) push(odd[t], 1);
+    if (order != 3) push(8, c8);
+    push(4, c4);
+    push(2, c2);
+    if (order == 3) push(8, c8);
+    if (order != 2)
+        for (int t = 0; t < no; t++) push(odd[t], 1);
+    int ns = 1;
+    for (int f = 0; f < P.nfac; f++) {
+        P.nslog[f] = (ns & (ns - 1)) == 0 ? __builtin_ctz(ns) : -1;
+        ns *= P.fac[f];
+    }
+    return P;
+}
+
 template <typename T2>
 __device__ __forceinline__ T2 cmul(T2 a, T2 b)
 {
@@ -1002,87 +1050,206 @@ __device__ __forceinline__ T2 cmul(T2 a, T2 b)
     return r;
 }
 template <typename T2>
-__device__ __forceinline__ T2 twid(const T2 *tw, int t, bool inv)
+__device__ __forceinline__ T2 cadd(T2 a, T2 b)
+{
+    T2 r;
+    r.x = a.x + b.x;
+    r.y = a.y + b.y;
+    return r;
+}
+template <typename T2>
+__device__ __forceinline__ T2 csub(T2 a, T2 b)
+{
+    T2 r;
+    r.x = a.x - b.x;
+    r.y = a.y - b.y;
+    return r;
+}
+// a -+ i b: the factor -i of a forward transform, +i of an inverse one
+template <bool INV, typename T2>
+__device__ __forceinline__ T2 csub_i(T2 a, T2 b)
+{
+    T2 r;
+    r.x = INV ? a.x - b.y : a.x + b.y;
+    r.y = INV ? a.y + b.x : a.y - b.x;
+    return r;
+}
+template <bool INV, typename T2>
+__device__ __forceinline__ T2 twid(const T2 *tw, int t)
 {
     T2 w = tw[t];
-    if (inv) w.y = -w.y;
+    if (INV) w.y = -w.y;
     return w;
+}
+
+// R-point DFTs in registers (R = 2, 3, 4, 5, 8), from their definitions
+template <int R, bool INV, typename T, typename T2>
+__device__ __forceinline__ void dft_small(T2 (&v)[R])
+{
+    if constexpr (R == 2) {
+        const T2 a = v[0], b = v[1];
+        v[0] = cadd(a, b);
+        v[1] = csub(a, b);
+    } else if constexpr (R == 3) {
+        const T s60 = T(0.86602540378443864676);  // sin(60 deg)
+        const T2 s = cadd(v[1], v[2]), d = csub(v[1], v[2]);
+        T2 m, e;
+        m.x = v[0].x - T(0.5) * s.x;
+        m.y = v[0].y - T(0.5) * s.y;
+        e.x = s60 * d.x;
+        e.y = s60 * d.y;
+        v[0] = cadd(v[0], s);
+        v[1] = csub_i<INV>(m, e);
+        v[2] = csub_i<!INV>(m, e);
+    } else if constexpr (R == 4) {
+        const T2 s02 = cadd(v[0], v[2]), d02 = csub(v[0], v[2]), s13 = cadd(v[1], v[3]), d13 = csub(v[1], v[3]);
+        v[0] = cadd(s02, s13);
+        v[1] = csub_i<INV>(d02, d13);
+        v[2] = csub(s02, s13);
+        v[3] = csub_i<!INV>(d02, d13);
+    } else if constexpr (R == 5) {
+        const T c1 = T(0.30901699437494742410), c2 = T(-0.80901699437494742410);  // cos 72, cos 144 deg
+        const T s1 = T(0.95105651629515357212), s2 = T(0.58778525229247312917);   // sin 72, sin 144 deg
+        const T2 sa = cadd(v[1], v[4]), da = csub(v[1], v[4]), sb = cadd(v[2], v[3]), db = csub(v[2], v[3]);
+        T2 m1, m2, e1, e2;
+        m1.x = v[0].x + c1 * sa.x + c2 * sb.x;
+        m1.y = v[0].y + c1 * sa.y + c2 * sb.y;
+        m2.x = v[0].x + c2 * sa.x + c1 * sb.x;
+        m2.y = v[0].y + c2 * sa.y + c1 * sb.y;
+        e1.x = s1 * da.x + s2 * db.x;
+        e1.y = s1 * da.y + s2 * db.y;
+        e2.x = s2 * da.x - s1 * db.x;
+        e2.y = s2 * da.y - s1 * db.y;
+        v[0] = cadd(v[0], cadd(sa, sb));
+        v[1] = csub_i<INV>(m1, e1);
+        v[4] = csub_i<!INV>(m1, e1);
+        v[2] = csub_i<INV>(m2, e2);
+        v[3] = csub_i<!INV>(m2, e2);
+    } else {
+        static_assert(R == 8, "radix");
+        const T r2 = T(0.70710678118654752440);
+        T2 e[4] = {cadd(v[0], v[4]), cadd(v[1], v[5]), cadd(v[2], v[6]), cadd(v[3], v[7])};
+        const T2 a = csub(v[0], v[4]), c = csub(v[1], v[5]), b = csub(v[2], v[6]), d = csub(v[3], v[7]);
+        const T2 f1 = csub_i<INV>(a, b), f3 = csub_i<!INV>(a, b), g1 = csub_i<INV>(c, d), g3 = csub_i<!INV>(c, d);
+        T2 h1, h3;  // the eighth roots: (1 -+ i)/sqrt 2 on g1, (-1 -+ i)/sqrt 2 on g3
+        h1.x = r2 * (INV ? g1.x - g1.y : g1.x + g1.y);
+        h1.y = r2 * (INV ? g1.y + g1.x : g1.y - g1.x);
+        h3.x = r2 * (INV ? -g3.x - g3.y : g3.y - g3.x);
+        h3.y = r2 * (INV ? g3.x - g3.y : -g3.x - g3.y);
+        dft_small<4, INV, T, T2>(e);
+        v[0] = e[0];
+        v[2] = e[1];
+        v[4] = e[2];
+        v[6] = e[3];
+        v[1] = cadd(f1, h1);
+        v[5] = csub(f1, h1);
+        v[3] = cadd(f3, h3);
+        v[7] = csub(f3, h3);
+    }
+}
+
+// one Stockham pass of radix R over every butterfly and line of the block
+template <int R, bool INV, typename T, typename T2>
+__device__ __forceinline__ void fft_pass(const T2 *a, T2 *b, int L, int N, int Ns, int nsl,
+                                         const T2 *__restrict__ tw, int ps)
+{
+    const int nb = N / R, ts = nb / Ns;
+    for (int j = threadIdx.y; j < nb; j += blockDim.y) {
+        int k, jb;
+        if (nsl >= 0) { k = j & (Ns - 1); jb = j >> nsl; }
+        else { jb = j / Ns; k = j - jb * Ns; }
+        const T2 *src = a + j * ps;
+        T2 *dst = b + (jb * Ns * R + k) * ps;
+        const int ss = nb * ps, ds = Ns * ps, kt = k * ts;
+        for (int l = threadIdx.x; l < L; l += blockDim.x) {
+            T2 v[R];
+#pragma unroll
+            for (int r = 0; r < R; r++) v[r] = src[r * ss + l];
+            if (Ns > 1) {
+#pragma unroll
+                for (int r = 1; r < R; r++) v[r] = cmul(v[r], twid<INV>(tw, r * kt));
+            }
+            dft_small<R, INV, T, T2>(v);
+#pragma unroll
+            for (int r = 0; r < R; r++) dst[r * ds + l] = v[r];
+        }
+    }
+}
+
+// a pass of any odd radix R (a prime factor above 5).  A butterfly owns its
+// inputs: its twiddled points become sums and differences x_r +- x_(R-r) in
+// place, and each pair of outputs m, R-m shares one cosine and one sine sum:
+// (R-1)^2 / 2 multiply-adds per component instead of 2 R^2, and no index
+// division: a 95 x 75 point periodic solve (radix 19) with its step went from
+// 1.88 to 1.42 ms per two steps.
+template <bool INV, typename T, typename T2>
+__device__ __forceinline__ void fft_pass_odd(T2 *a, T2 *b, int L, int N, int R, int Ns, int nsl,
+                                             const T2 *__restrict__ tw, int ps)
+{
+    const int nb = N / R, ts = nb / Ns, H = (R - 1) / 2;
+    for (int j = threadIdx.y; j < nb; j += blockDim.y) {
+        int k, jb;
+        if (nsl >= 0) { k = j & (Ns - 1); jb = j >> nsl; }
+        else { jb = j / Ns; k = j - jb * Ns; }
+        T2 *src = a + j * ps;
+        T2 *dst = b + (jb * Ns * R + k) * ps;
+        const int ss = nb * ps, ds = Ns * ps, kt = k * ts;
+        for (int l = threadIdx.x; l < L; l += blockDim.x) {
+            const T2 v0 = src[l];
+            T2 sum = v0;
+            for (int r = 1; r <= H; r++) {
+                T2 u = src[r * ss + l], w = src[(R - r) * ss + l];
+                if (Ns > 1) {
+                    u = cmul(u, twid<INV>(tw, r * kt));
+                    w = cmul(w, twid<INV>(tw, (R - r) * kt));
+                }
+                const T2 s = cadd(u, w);
+                src[r * ss + l] = s;
+                src[(R - r) * ss + l] = csub(u, w);
+                sum = cadd(sum, s);
+            }
+            dst[l] = sum;
+            for (int m = 1; m <= H; m++) {
+                T2 c = v0, e;
+                e.x = T(0);
+                e.y = T(0);
+                int t = 0;
+                for (int r = 1; r <= H; r++) {
+                    t += m * nb;  // (r m mod R) nb
+                    if (t >= N) t -= N;
+                    const T2 w = tw[t];
+                    const T2 s = src[r * ss + l], d = src[(R - r) * ss + l];
+                    c.x += s.x * w.x;
+                    c.y += s.y * w.x;
+                    e.x -= d.x * w.y;  // tw holds -sin
+                    e.y -= d.y * w.y;
+                }
+                dst[m * ds + l] = csub_i<INV>(c, e);
+                dst[(R - m) * ds + l] = csub_i<!INV>(c, e);
+            }
+        }
+    }
 }
 
 // Batched shared-memory FFT.  L lines; element (point n, line l) lives at
 // buf[n*ps + l] with ps >= L (padding keeps a thread that walks one line
 // across points off a single bank).  Threads are 2-D: x runs over lines,
 // y over the butterflies of a pass, so no index needs a division by L.
-template <typename T, typename T2>
-__device__ T2 *fft_smem(T2 *a, T2 *b, int L, const FftPlan &P, const T2 *__restrict__ tw, bool inv, int ps)
+// A pass costs a round trip through shared memory and a barrier, so the plan
+// takes radix 8 first: 512 points are three passes where radix 4 takes five.
+template <bool INV, typename T, typename T2>
+__device__ T2 *fft_smem(T2 *a, T2 *b, int L, const FftPlan &P, const T2 *__restrict__ tw, int ps)
 {
     const int N = P.n;
     int Ns = 1;
     for (int f = 0; f < P.nfac; ++f) {
-        const int R = P.fac[f];
-        const int nb = N / R;
-        const int ts = N / (Ns * R);
-        const int nsl = P.nslog[f];
-        for (int j = threadIdx.y; j < nb; j += blockDim.y) {
-            int k, jb;
-            if (nsl >= 0) { k = j & (Ns - 1); jb = j >> nsl; }
-            else { k = j % Ns; jb = j / Ns; }
-            const int ob = jb * Ns * R + k;
-            for (int l = threadIdx.x; l < L; l += blockDim.x) {
-                if (R == 2) {
-                    T2 v0 = a[j * ps + l];
-                    T2 v1 = a[(j + nb) * ps + l];
-                    if (k) v1 = cmul(v1, twid(tw, k * ts, inv));
-                    T2 s, d;
-                    s.x = v0.x + v1.x; s.y = v0.y + v1.y;
-                    d.x = v0.x - v1.x; d.y = v0.y - v1.y;
-                    b[ob * ps + l] = s;
-                    b[(ob + Ns) * ps + l] = d;
-                } else if (R == 4) {
-                    T2 v0 = a[j * ps + l];
-                    T2 v1 = a[(j + nb) * ps + l];
-                    T2 v2 = a[(j + 2 * nb) * ps + l];
-                    T2 v3 = a[(j + 3 * nb) * ps + l];
-                    if (k) {
-                        v1 = cmul(v1, twid(tw, k * ts, inv));
-                        v2 = cmul(v2, twid(tw, 2 * k * ts, inv));
-                        v3 = cmul(v3, twid(tw, 3 * k * ts, inv));
-                    }
-                    T2 s02, d02, s13, d13, x0, x1, x2, x3;
-                    s02.x = v0.x + v2.x; s02.y = v0.y + v2.y;
-                    d02.x = v0.x - v2.x; d02.y = v0.y - v2.y;
-                    s13.x = v1.x + v3.x; s13.y = v1.y + v3.y;
-                    d13.x = v1.x - v3.x; d13.y = v1.y - v3.y;
-                    x0.x = s02.x + s13.x; x0.y = s02.y + s13.y;
-                    x2.x = s02.x - s13.x; x2.y = s02.y - s13.y;
-                    if (!inv) {  // X1 = d02 - i d13, X3 = d02 + i d13
-                        x1.x = d02.x + d13.y; x1.y = d02.y - d13.x;
-                        x3.x = d02.x - d13.y; x3.y = d02.y + d13.x;
-                    } else {
-                        x1.x = d02.x - d13.y; x1.y = d02.y + d13.x;
-                        x3.x = d02.x + d13.y; x3.y = d02.y - d13.x;
-                    }
-                    b[ob * ps + l] = x0;
-                    b[(ob + Ns) * ps + l] = x1;
-                    b[(ob + 2 * Ns) * ps + l] = x2;
-                    b[(ob + 3 * Ns) * ps + l] = x3;
-                } else {  // generic radix: direct R-point DFT with combined twiddles
-                    for (int m = 0; m < R; ++m) {
-                        T2 acc;
-                        acc.x = T(0);
-                        acc.y = T(0);
-                        for (int r = 0; r < R; ++r) {
-                            const int t = (k * r * ts + ((r * m) % R) * nb) % N;
-                            T2 x = a[(j + r * nb) * ps + l];
-                            T2 wv = twid(tw, t, inv);
-                            acc.x += x.x * wv.x - x.y * wv.y;
-                            acc.y += x.x * wv.y + x.y * wv.x;
-                        }
-                        b[(ob + m * Ns) * ps + l] = acc;
-                    }
-                }
-            }
-        }
+        const int R = P.fac[f], nsl = P.nslog[f];
+        if (R == 8) fft_pass<8, INV, T, T2>(a, b, L, N, Ns, nsl, tw, ps);
+        else if (R == 4) fft_pass<4, INV, T, T2>(a, b, L, N, Ns, nsl, tw, ps);
+        else if (R == 2) fft_pass<2, INV, T, T2>(a, b, L, N, Ns, nsl, tw, ps);
+        else if (R == 3) fft_pass<3, INV, T, T2>(a, b, L, N, Ns, nsl, tw, ps);
+        else if (R == 5) fft_pass<5, INV, T, T2>(a, b, L, N, Ns, nsl, tw, ps);
+        else fft_pass_odd<INV, T, T2>(a, b, L, N, R, Ns, nsl, tw, ps);
         __syncthreads();
         T2 *tmp = a;
         a = b;
@@ -1090,6 +1257,117 @@ __device__ T2 *fft_smem(T2 *a, T2 *b, int L, const FftPlan &P, const T2 *__restr
         Ns *= R;
     }
     return a;
+}
+
+// ---------------------------------------------------------------------------
+// The spectral buffer.  The divergence is real, so its transform along y is
+// Hermitian and only the wavenumbers q = 0 .. nj/2 are stored, transformed
+// along x and solved; the inverse transform rebuilds the rest.  Element
+// (x-index i, wavenumber q, level k = 1 .. NZ-2) lives at
+// (i*nh + q)*nzs + k - 1, rows of whole 32-byte sectors.  A y transform
+// carries two adjacent levels, 1+2l and 2+2l, as the real and imaginary part
+// of one complex line.  Against full complex transforms that halves the
+// spectral traffic, the x transforms, the vertical solves and the y
+// transforms' lines.  With the radix-8 passes: FP32 squall line 512x512x64
+// 12.49 -> 10.46 ms per two steps, uneven ensemble (96 and 160 points, radix
+// 3 and 5) 81.9 -> 67.4 ms per 20 steps with download, FP64 thunderstorm
+// 128x128x48 9.70 -> 9.05 ms per two steps.
+// ---------------------------------------------------------------------------
+__host__ __device__ constexpr int spec_nh(int nj) { return nj / 2 + 1; }
+__host__ __device__ constexpr int spec_nzs(int nz) { return (nz - 2 + 3) & ~3; }
+__host__ __device__ constexpr int level_pairs(int nz) { return (nz - 1) / 2; }
+// point stride of KT transform lines (odd: a butterfly's strided points fall
+// on different banks) and the two buffers of n points
+__host__ __device__ constexpr int fft_ps(int kt) { return kt | 1; }
+__host__ __device__ constexpr size_t fft_bytes(int n, int kt, size_t elem) { return 2 * (size_t)n * fft_ps(kt) * elem; }
+template <typename T>
+__device__ __forceinline__ long spec_at(const KParams<T> &p, int i, int q, int k)
+{
+    return ((long)i * p.nh + q) * p.nzs + k - 1;
+}
+
+// two adjacent levels' spectra to the buffer (16-byte aligned in FP32: the
+// level index is odd and rows are multiples of four levels)
+template <typename T2>
+__device__ __forceinline__ void st_pair(T2 *dst, T2 a, T2 b)
+{
+    if constexpr (sizeof(T2) == 8) {
+        *reinterpret_cast<float4 *>(dst) = make_float4(a.x, a.y, b.x, b.y);
+    } else {
+        dst[0] = a;
+        dst[1] = b;
+    }
+}
+template <typename T2>
+__device__ __forceinline__ void ld_pair(const T2 *src, T2 &a, T2 &b)
+{
+    if constexpr (sizeof(T2) == 8) {
+        const float4 v = *reinterpret_cast<const float4 *>(src);
+        a.x = v.x;
+        a.y = v.y;
+        b.x = v.z;
+        b.y = v.w;
+    } else {
+        a = src[0];
+        b = src[1];
+    }
+}
+
+// forward transform along y of the level-pair lines in `a` (KT lines from
+// line l0, free buffer b) and the half spectra of both levels to row `is`
+template <typename T>
+__device__ __forceinline__ void fft_y_store(const KParams<T> &p, typename V2<T>::t *a, typename V2<T>::t *b,
+                                            typename V2<T>::t *spec, const FftPlan &pj,
+                                            const typename V2<T>::t *tw, int KT, int is, int l0)
+{
+    typedef typename V2<T>::t T2;
+    const int ps = fft_ps(KT), lt = min(KT, level_pairs(p.nz) - l0);
+    const T2 *r = fft_smem<false, T, T2>(a, b, KT, pj, tw, ps);
+    for (int q = threadIdx.y; q < p.nh; q += blockDim.y)
+        for (int l = threadIdx.x; l < lt; l += blockDim.x) {
+            const T2 z = r[q * ps + l], c = r[(q ? p.nj - q : 0) * ps + l];
+            T2 u, w;  // (Z_q + conj Z_-q)/2 and (Z_q - conj Z_-q)/(2i)
+            u.x = T(0.5) * (z.x + c.x);
+            u.y = T(0.5) * (z.y - c.y);
+            w.x = T(0.5) * (z.y + c.y);
+            w.y = T(0.5) * (c.x - z.x);
+            st_pair(spec + spec_at(p, is, q, 1 + 2 * (l0 + l)), u, w);
+        }
+}
+// the inverse: half spectra of row `is` into level-pair lines, transformed;
+// returns the buffer whose .x and .y are the two levels' real values
+template <typename T>
+__device__ __forceinline__ typename V2<T>::t *fft_y_load(const KParams<T> &p, typename V2<T>::t *a,
+                                                         typename V2<T>::t *b, const typename V2<T>::t *spec,
+                                                         const FftPlan &pj, const typename V2<T>::t *tw, int KT,
+                                                         int is, int l0)
+{
+    typedef typename V2<T>::t T2;
+    const int ps = fft_ps(KT), np = level_pairs(p.nz);
+#pragma unroll 4
+    for (int q = threadIdx.y; q < p.nh; q += blockDim.y)
+        for (int l = threadIdx.x; l < KT; l += blockDim.x) {
+            T2 u, w;
+            u.x = u.y = w.x = w.y = T(0);
+            const int k = 1 + 2 * (l0 + l);
+            if (l0 + l < np) ld_pair(spec + spec_at(p, is, q, k), u, w);
+            if (k + 1 > p.nz - 2) w.x = w.y = T(0);  // an odd level count's padding
+            T2 z, c;
+            if (q == 0 || 2 * q == p.nj) {  // real wavenumbers
+                z.x = u.x;
+                z.y = w.x;
+                a[q * ps + l] = z;
+            } else {
+                z.x = u.x - w.y;
+                z.y = u.y + w.x;
+                c.x = u.x + w.y;
+                c.y = w.x - u.y;
+                a[q * ps + l] = z;
+                a[(p.nj - q) * ps + l] = c;
+            }
+        }
+    __syncthreads();
+    return fft_smem<true, T, T2>(a, b, KT, pj, tw, ps);
 }
 
 // divergence tendency of the pressure equation at a physical point
@@ -1108,18 +1386,17 @@ __device__ __forceinline__ T divergence(const KParams<T> &p, const KFields<T> &F
 
 // divergence (with the mirror / periodic placement of divergence3d and
 // divergence3d_periodic) + forward FFT along y.  Block = (spectral row i,
-// tile of KT levels starting at level 1).
+// tile of KT level pairs).
 template <typename T>
 __device__ void div_fft_y_body(const KParams<T> &p, const KFields<T> &F, typename V2<T>::t *spec, const FftPlan &pj,
                                const typename V2<T>::t *tw, T sdt, int KT, int bx, int by)
 {
     typedef typename V2<T>::t T2;
     extern __shared__ unsigned char smem_raw[];
+    const int ps = fft_ps(KT);
     T2 *a = (T2 *)smem_raw;
-    T2 *b = a + (long)p.nj * KT;
-    const int is = bx;
-    const int k0 = 1 + by * KT;
-    const int kt = min(KT, p.nz - 1 - k0);
+    T2 *b = a + (long)p.nj * ps;
+    const int is = bx, l0 = by * KT;
     int ii;
     if (!p.periodic) ii = min(max(is, 1), p.nx - 2);
     else ii = is + 3;
@@ -1131,17 +1408,13 @@ __device__ void div_fft_y_body(const KParams<T> &p, const KFields<T> &F, typenam
             T2 v;
             v.y = T(0);
             v.x = T(0);
-            if (l < kt) {
-                const int jj = min(max(q, 1), p.ny - 2);
-                v.x = divergence(p, F, ii, jj, k0 + l, sdt);
-            }
-            a[q * KT + l] = v;
+            const int jj = min(max(q, 1), p.ny - 2), k = 1 + 2 * (l0 + l);
+            if (k < p.nz - 1) v.x = divergence(p, F, ii, jj, k, sdt);
+            if (k + 1 < p.nz - 1) v.y = divergence(p, F, ii, jj, k + 1, sdt);
+            a[q * ps + l] = v;
         }
     __syncthreads();
-    T2 *r = fft_smem<T, T2>(a, b, KT, pj, tw, false, KT);
-    for (int q = threadIdx.y; q < p.nj; q += blockDim.y)
-        for (int l = threadIdx.x; l < kt; l += blockDim.x)
-            spec[((long)is * p.nj + q) * p.nz + k0 + l] = r[q * KT + l];
+    fft_y_store(p, a, b, spec, pj, tw, KT, is, l0);
 }
 template <typename T>
 __global__ void k_div_fft_y(KParams<T> p, KFields<T> F, typename V2<T>::t *spec, FftPlan pj,
@@ -1158,18 +1431,20 @@ __device__ void fft_x_body(const KParams<T> &p, typename V2<T>::t *spec, const F
 {
     typedef typename V2<T>::t T2;
     extern __shared__ unsigned char smem_raw[];
+    const int ps = fft_ps(KT);
     T2 *a = (T2 *)smem_raw;
-    T2 *b = a + (long)p.ni * KT;
+    T2 *b = a + (long)p.ni * ps;
     const int k0 = 1 + bx * KT;
     const int kt = min(KT, p.nz - 1 - k0);
+    T2 *g = spec + spec_at(p, 0, q, k0);
+    const long gs = (long)p.nh * p.nzs;
     for (int i = threadIdx.y; i < p.ni; i += blockDim.y)
         for (int l = threadIdx.x; l < KT; l += blockDim.x)
-            cp_elem(a + i * KT + l, spec + ((long)i * p.nj + q) * p.nz + k0 + min(l, kt - 1), l < kt);
+            cp_elem(a + i * ps + l, g + i * gs + min(l, kt - 1), l < kt);
     cp_wait_all_sync();
-    T2 *r = fft_smem<T, T2>(a, b, KT, pi, tw, inv != 0, KT);
+    const T2 *r = inv ? fft_smem<true, T, T2>(a, b, KT, pi, tw, ps) : fft_smem<false, T, T2>(a, b, KT, pi, tw, ps);
     for (int i = threadIdx.y; i < p.ni; i += blockDim.y)
-        for (int l = threadIdx.x; l < kt; l += blockDim.x)
-            spec[((long)i * p.nj + q) * p.nz + k0 + l] = r[i * KT + l];
+        for (int l = threadIdx.x; l < kt; l += blockDim.x) g[i * gs + l] = r[i * ps + l];
 }
 // the level tiles of a wavenumber run next to each other (shared rows)
 template <typename T>
@@ -1243,20 +1518,35 @@ __device__ __forceinline__ void thomas_column_fast(float2 *x, float *Fw, int nz,
     float Fk = cc[1] * z;
     Fw[1] = Fk;
     float xr = x[1].x * inv_size2d * z, xi = x[1].y * inv_size2d * z;
+    // the next level's values are read before this level's are written, so
+    // the loads stay off the recurrence
+    float2 d = x[2];
+    float rk = rhou[2], ak = ac[2], ck = cc[2], vk = vc[2];
     x[1] = make_float2(xr, xi);
     for (int k = 2; k < nz - 1; k++) {
-        z = __frcp_rn(rhou[k] * hb - vc[k] - ac[k] * Fk);
-        Fk = cc[k] * z;
+        const float2 dn = x[min(k + 1, nz - 2)];
+        const float rn = rhou[k + 1], an = ac[k + 1], cn = cc[k + 1], vn = vc[k + 1];
+        z = __frcp_rn(rk * hb - vk - ak * Fk);
+        Fk = ck * z;
         Fw[k] = Fk;
-        xr = (x[k].x * inv_size2d - ac[k] * xr) * z;
-        xi = (x[k].y * inv_size2d - ac[k] * xi) * z;
+        xr = (d.x * inv_size2d - ak * xr) * z;
+        xi = (d.y * inv_size2d - ak * xi) * z;
         x[k] = make_float2(xr, xi);
+        d = dn;
+        rk = rn; ak = an; ck = cn; vk = vn;
     }
     if (gauge) { xr = 0.f; xi = 0.f; x[nz - 2] = make_float2(0.f, 0.f); }
+    d = x[nz - 3];
+    float f = Fw[nz - 3];
     for (int k = nz - 3; k >= 1; k--) {
-        xr = x[k].x - Fw[k] * xr;
-        xi = x[k].y - Fw[k] * xi;
+        const int km = max(k - 1, 1);
+        const float2 dn = x[km];
+        const float fn = Fw[km];
+        xr = d.x - f * xr;
+        xi = d.y - f * xi;
         x[k] = make_float2(xr, xi);
+        d = dn;
+        f = fn;
     }
 }
 
@@ -1391,15 +1681,30 @@ __device__ void mean_mode_solve_T(T2 *x, int nl, const double *__restrict__ Minv
 }
 
 // true for the low horizontal wavenumbers solved in FP64 in FP32 contexts
+// (q <= nj/2 is its own distance from 0)
 template <typename T>
-__device__ __forceinline__ bool low_mode(const KParams<T> &p, long col)
+__device__ __forceinline__ bool low_mode(const KParams<T> &p, int pp, int q)
 {
-    if (p.low_modes <= 0) return false;
-    const int pp = (int)(col / p.nj), qq = (int)(col % p.nj);
-    return min(pp, p.ni - pp) < p.low_modes && min(qq, p.nj - qq) < p.low_modes;
+    return min(pp, p.ni - pp) < p.low_modes && q < p.low_modes;
 }
 
-// columns bx*TC .. of the spectral buffer
+// stage nc spectral columns of nl levels (row stride rs) into shared columns
+// of stride cs, a warp per column; and back
+template <typename T2>
+__device__ __forceinline__ void columns_in(T2 *xs, int cs, const T2 *g, int rs, int nc, int nl)
+{
+    for (int c = threadIdx.x >> 5; c < nc; c += blockDim.x >> 5)
+        for (int l = threadIdx.x & 31; l < nl; l += 32) cp_elem(xs + c * cs + l, g + (long)c * rs + l, true);
+    cp_wait_all_sync();
+}
+template <typename T2>
+__device__ __forceinline__ void columns_out(const T2 *xs, int cs, T2 *g, int rs, int nc, int nl)
+{
+    for (int c = threadIdx.x >> 5; c < nc; c += blockDim.x >> 5)
+        for (int l = threadIdx.x & 31; l < nl; l += 32) g[(long)c * rs + l] = xs[c * cs + l];
+}
+
+// columns bx*TC .. of the spectral buffer (blocks of whole warps)
 template <typename T>
 __device__ void thomas_body(const KParams<T> &p, typename V2<T>::t *spec, int TC, long bx)
 {
@@ -1409,43 +1714,45 @@ __device__ void thomas_body(const KParams<T> &p, typename V2<T>::t *spec, int TC
     const int cs = p.nz | 1;  // odd column stride: no bank conflicts between columns
     T2 *xs = (T2 *)smem_raw;
     T *fs = (T *)(xs + (long)TC * cs);
-    const long ncol = (long)p.ni * p.nj;
-    const long c0 = bx * TC;
-    const int nc = (int)min((long)TC, ncol - c0);
-    T2 *g = spec + c0 * p.nz;
-    for (int w = threadIdx.x; w < nc * p.nz; w += blockDim.x) cp_elem(xs + (w / p.nz) * cs + w % p.nz, g + w, true);
-    cp_wait_all_sync();
+    const int ncol = p.ni * p.nh, nl = p.nz - 2;
+    const int c0 = (int)bx * TC;
+    const int nc = min(TC, ncol - c0);
+    T2 *g = spec + (long)c0 * p.nzs;
+    columns_in(xs, cs, g, p.nzs, nc, nl);
     const double size2d = (double)(p.ni * p.nj);
+    bool any_low = false;
     for (int c = threadIdx.x; c < nc; c += blockDim.x) {
-        const long col = c0 + c;
+        const int col = c0 + c, pp = col / p.nh, q = col - pp * p.nh;
+        T2 *x = xs + (long)c * cs - 1;
         if (sizeof(T) == 8) {
             double Floc[PPM_MAXZ];
-            thomas_column<T, double>(p, xs + (long)c * cs, Floc, col, size2d, p.rhou_d, p.acoef_d, p.ccoef_d,
-                                     p.vcoef_d);
-        } else if (!low_mode(p, col)) {
+            thomas_column<T, double>(p, x, Floc, col, size2d, p.rhou_d, p.acoef_d, p.ccoef_d, p.vcoef_d);
+        } else if (!low_mode(p, pp, q)) {
             const float hb = 2.0f * (float)p.hcoef[col] / (float)p.dx2;
-            thomas_column_fast((float2 *)(xs + (long)c * cs), (float *)(fs + (long)c * cs), p.nz, hb,
-                               (float)(1.0 / size2d), (const float *)p.rhou, (const float *)p.acoef,
-                               (const float *)p.ccoef, (const float *)p.vcoef, col == 0);
+            thomas_column_fast((float2 *)x, (float *)(fs + (long)c * cs), p.nz, hb, (float)(1.0 / size2d),
+                               (const float *)p.rhou, (const float *)p.acoef, (const float *)p.ccoef,
+                               (const float *)p.vcoef, col == 0);
+        } else {
+            any_low = true;
         }
     }
-    if (sizeof(T) != 8 && p.low_modes > 0) {
+    if (sizeof(T) != 8 && p.low_modes > 0 && __syncthreads_or(any_low)) {
         const int warp = threadIdx.x >> 5;
         if (warp == 0) {  // the low modes of this block, one after the other
             for (int c = 0; c < nc; c++) {
-                const long col = c0 + c;
-                if (!low_mode(p, col) || (col == 0 && p.mean_inv)) continue;
-                pcr_column_f64(xs + (long)c * cs, p.nz - 2, p.hcoef[col], p.dx2, size2d, p.rhou_d, p.acoef_d,
+                const int col = c0 + c, pp = col / p.nh;
+                if (!low_mode(p, pp, col - pp * p.nh) || (col == 0 && p.mean_inv)) continue;
+                pcr_column_f64(xs + (long)c * cs - 1, nl, p.hcoef[col], p.dx2, size2d, p.rhou_d, p.acoef_d,
                                p.ccoef_d, p.vcoef_d, col == 0, pcr_wk);
             }
         }
         if (c0 == 0 && p.mean_inv) {  // the mean mode: block-wide, after warp 0's reductions
             __syncthreads();
-            mean_mode_solve(xs, p.nz - 2, p.mean_inv, size2d, pcr_wk);
+            mean_mode_solve(xs - 1, nl, p.mean_inv, size2d, pcr_wk);
         }
     }
     __syncthreads();
-    for (int w = threadIdx.x; w < nc * p.nz; w += blockDim.x) g[w] = xs[(w / p.nz) * cs + w % p.nz];
+    columns_out(xs, cs, g, p.nzs, nc, nl);
 }
 template <typename T>
 __global__ void k_thomas(KParams<T> p, typename V2<T>::t *spec, int TC)
@@ -1473,16 +1780,15 @@ __device__ void spectral_x_body(const KParams<T> &p, typename V2<T>::t *spec, co
     }
     for (int i = threadIdx.y; i < p.ni; i += blockDim.y)
         for (int l = threadIdx.x; l < nl; l += blockDim.x)
-            cp_elem(a + i * ps + l, spec + ((long)i * p.nj + q) * p.nz + 1 + l, true);
+            cp_elem(a + i * ps + l, spec + spec_at(p, i, q, 1 + l), true);
     cp_wait_all_sync();
-    T2 *r = fft_smem<T, T2>(a, b, nl, pi, tw, false, ps);
+    T2 *r = fft_smem<false, T, T2>(a, b, nl, pi, tw, ps);
     T2 *fr = (r == a) ? b : a;  // free buffer: holds the Thomas coefficients
     const double size2d = (double)(p.ni * p.nj);
-    const int aq = min(q, p.nj - q);
-    const bool q_low = p.low_modes > 0 && aq < p.low_modes;
+    const bool q_low = p.low_modes > 0 && q < p.low_modes;
     if (sizeof(T) == 8) {  // parity path: the reference's Thomas recurrence in FP64
         for (int pp = tid; pp < p.ni; pp += nth) {
-            const long col = (long)pp * p.nj + q;
+            const long col = (long)pp * p.nh + q;
             double *Fw = (double *)(fr + (long)pp * ps) - 1;
             thomas_column<T, double>(p, r + (long)pp * ps - 1, Fw, col, size2d, d_r, d_a, d_c, d_v);
         }
@@ -1491,7 +1797,7 @@ __device__ void spectral_x_body(const KParams<T> &p, typename V2<T>::t *spec, co
         for (int pp = tid; pp < p.ni; pp += nth) {
             const int ap = min(pp, p.ni - pp);
             if (q_low && ap < p.low_modes) continue;  // FP64 islands below
-            const long col = (long)pp * p.nj + q;
+            const long col = (long)pp * p.nh + q;
             const float hb = 2.0f * (float)p.hcoef[col] / dx2;
             float *Fw = (float *)(fr + (long)pp * ps) - 1;
             thomas_column_fast((float2 *)(r + (long)pp * ps - 1), Fw, p.nz, hb, inv_s, (const float *)c_r,
@@ -1507,7 +1813,7 @@ __device__ void spectral_x_body(const KParams<T> &p, typename V2<T>::t *spec, co
                 }
                 for (int w = 0; w < nis; w++) {
                     const int pp = islands[w];
-                    const long col = (long)pp * p.nj + q;
+                    const long col = (long)pp * p.nh + q;
                     if (col == 0 && p.mean_inv) continue;
                     pcr_column_f64(r + (long)pp * ps - 1, nl, p.hcoef[col], p.dx2, size2d, d_r, d_a, d_c, d_v,
                                    col == 0, pcr_wk);
@@ -1520,9 +1826,9 @@ __device__ void spectral_x_body(const KParams<T> &p, typename V2<T>::t *spec, co
         }
     }
     __syncthreads();
-    T2 *o = fft_smem<T, T2>(r, fr, nl, pi, tw, true, ps);
+    T2 *o = fft_smem<true, T, T2>(r, fr, nl, pi, tw, ps);
     for (int i = threadIdx.y; i < p.ni; i += blockDim.y)
-        for (int l = threadIdx.x; l < nl; l += blockDim.x) spec[((long)i * p.nj + q) * p.nz + 1 + l] = o[i * ps + l];
+        for (int l = threadIdx.x; l < nl; l += blockDim.x) spec[spec_at(p, i, q, 1 + l)] = o[i * ps + l];
 }
 template <typename T>
 __global__ void k_spectral_x(KParams<T> p, typename V2<T>::t *spec, FftPlan pi, const typename V2<T>::t *tw,
@@ -1547,46 +1853,51 @@ __device__ void ifft_y_pi_body(const KParams<T> &p, const KFields<T> &F, typenam
 {
     typedef typename V2<T>::t T2;
     extern __shared__ unsigned char smem_raw[];
+    const int ps = fft_ps(KT);
     T2 *a = (T2 *)smem_raw;
-    T2 *b = a + (long)p.nj * KT;
-    const int is = bx;
-    const int k0 = 1 + by * KT;
-    const int kt = min(KT, p.nz - 1 - k0);
-    for (int q = threadIdx.y; q < p.nj; q += blockDim.y)
-        for (int l = threadIdx.x; l < KT; l += blockDim.x)
-            cp_elem(a + q * KT + l, spec + ((long)is * p.nj + q) * p.nz + k0 + min(l, kt - 1), l < kt);
-    cp_wait_all_sync();
-    T2 *r = fft_smem<T, T2>(a, b, KT, pj, tw, true, KT);
+    T2 *b = a + (long)p.nj * ps;
+    const int is = bx, l0 = by * KT;
+    const int lt = min(KT, level_pairs(p.nz) - l0);
+    const T2 *r = fft_y_load(p, a, b, spec, pj, tw, KT, is, l0);
     T *PI = F.pi;
     const int nz = p.nz, ny = p.ny;
     for (int j = threadIdx.y; j < p.nj; j += blockDim.y)
-      for (int l = threadIdx.x; l < kt; l += blockDim.x) {
-        const int w = j * KT + l;
-        const int k = k0 + l;
+      for (int l = threadIdx.x; l < lt; l += blockDim.x) {
+        const T2 raw = r[j * ps + l];
         if (!p.periodic) {
             const int i = is;
             // levels 1..NZ-2: mirrored in x and y
-            const T v = r[min(max(j, 1), ny - 2) * KT + l].x;
-            if (i >= 1 && i <= p.nx - 2) {
-                PI[gix(ny, nz, i, j, k)] = v;
-                if (i == 1) PI[gix(ny, nz, 0, j, k)] = v;
-                if (i == p.nx - 2) PI[gix(ny, nz, p.nx - 1, j, k)] = v;
+            const T2 mir = r[min(max(j, 1), ny - 2) * ps + l];
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const int k = 1 + 2 * (l0 + l) + h;
+                if (k > nz - 2) break;
+                const T v = h ? mir.y : mir.x, w = h ? raw.y : raw.x;
+                if (i >= 1 && i <= p.nx - 2) {
+                    PI[gix(ny, nz, i, j, k)] = v;
+                    if (i == 1) PI[gix(ny, nz, 0, j, k)] = v;
+                    if (i == p.nx - 2) PI[gix(ny, nz, p.nx - 1, j, k)] = v;
+                }
+                // levels 0 and NZ-1: raw copies of levels 1 and NZ-2
+                if (k == 1) PI[gix(ny, nz, i, j, 0)] = w;
+                if (k == nz - 2) PI[gix(ny, nz, i, j, nz - 1)] = w;
             }
-            // levels 0 and NZ-1: raw copies of levels 1 and NZ-2
-            const T raw = r[w].x;
-            if (k == 1) PI[gix(ny, nz, i, j, 0)] = raw;
-            if (k == nz - 2) PI[gix(ny, nz, i, j, nz - 1)] = raw;
         } else {
             const int i = is + 3;
-            const T raw = r[w].x;
             int dst[2] = {i, -1};
             if (i >= p.nx - 6 && i <= p.nx - 4) dst[1] = i - (p.nx - 6);
             if (i >= 3 && i <= 5) dst[1] = p.nx - 3 + (i - 3);
-            for (int d = 0; d < 2; d++) {
-                if (dst[d] < 0) continue;
-                PI[gix(ny, nz, dst[d], j, k)] = raw;
-                if (k == 1) PI[gix(ny, nz, dst[d], j, 0)] = raw;
-                if (k == nz - 2) PI[gix(ny, nz, dst[d], j, nz - 1)] = raw;
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const int k = 1 + 2 * (l0 + l) + h;
+                if (k > nz - 2) break;
+                const T w = h ? raw.y : raw.x;
+                for (int d = 0; d < 2; d++) {
+                    if (dst[d] < 0) continue;
+                    PI[gix(ny, nz, dst[d], j, k)] = w;
+                    if (k == 1) PI[gix(ny, nz, dst[d], j, 0)] = w;
+                    if (k == nz - 2) PI[gix(ny, nz, dst[d], j, nz - 1)] = w;
+                }
             }
         }
     }

@@ -263,24 +263,22 @@ struct Lin : LinBase {
     void adj_pressure(double st)
     {
         KFields<T> A = fields();
-        const int nkt_y = cdiv(e.NZ - 2, e.KTy), nkt_x = cdiv(e.NZ - 2, e.KTx);
-        const dim3 by_y(e.KTy, std::max(1, 256 / e.KTy)), by_x(e.KTx, std::max(1, 256 / e.KTx));
         cudaStream_t s = e.stream;
-        k_adj_fft_y_in<T><<<dim3(nkt_y, e.kp.ni), by_y, e.smem_y, s>>>(e.kp, lpi_f, e.spec, e.plan_j, e.tw_j, e.KTy);
+        k_adj_fft_y_in<T><<<e.grid_y(), e.block_y(), e.smem_y, s>>>(e.kp, lpi_f, e.spec, e.plan_j, e.tw_j, e.KTy);
         if (e.psx > 0) {  // x transforms and the solves fused, as in the forward step
             // the adjoint kernel's registers allow blocks of up to 512 threads
             const int nl = e.NZ - 2, bx = std::min(nl, 64), nt = std::min(e.sx_threads, 512);
-            k_spectral_x_adj<T><<<e.kp.nj, dim3(bx, std::max(1, nt / bx)), e.smem_sx, s>>>(e.kp, e.spec, e.plan_i,
+            k_spectral_x_adj<T><<<e.kp.nh, dim3(bx, std::max(1, nt / bx)), e.smem_sx, s>>>(e.kp, e.spec, e.plan_i,
                                                                                          e.tw_i, e.psx);
             e.launches += 1;
         } else {
-            k_fft_x<T><<<dim3(nkt_x, e.kp.nj), by_x, e.smem_x, s>>>(e.kp, e.spec, e.plan_i, e.tw_i, 0, e.KTx);
-            const long ncol = (long)e.kp.ni * e.kp.nj;
+            k_fft_x<T><<<e.grid_x(), e.block_x(), e.smem_x, s>>>(e.kp, e.spec, e.plan_i, e.tw_i, 0, e.KTx);
+            const long ncol = (long)e.kp.ni * e.kp.nh;
             k_thomas_adj<T><<<cdiv(ncol, e.TC), 256, e.smem_th, s>>>(e.kp, e.spec, e.TC);
-            k_fft_x<T><<<dim3(nkt_x, e.kp.nj), by_x, e.smem_x, s>>>(e.kp, e.spec, e.plan_i, e.tw_i, 1, e.KTx);
+            k_fft_x<T><<<e.grid_x(), e.block_x(), e.smem_x, s>>>(e.kp, e.spec, e.plan_i, e.tw_i, 1, e.KTx);
             e.launches += 3;
         }
-        k_adj_ifft_y_out<T><<<dim3(nkt_y, e.kp.ni), by_y, e.smem_y, s>>>(e.kp, e.spec, dbar, e.plan_j, e.tw_j, e.KTy);
+        k_adj_ifft_y_out<T><<<e.grid_y(), e.block_y(), e.smem_y, s>>>(e.kp, e.spec, dbar, e.plan_j, e.tw_j, e.KTy);
         bool div_quad = false;
         if constexpr (sizeof(T) == 4) div_quad = adj_quad;
         if (div_quad) {

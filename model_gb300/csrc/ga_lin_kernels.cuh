@@ -750,7 +750,7 @@ __global__ void __launch_bounds__(AJ_THREADS, sizeof(T) == 4 ? 3 : 2)
     k_adj_advect(KParams<T> p, const T *__restrict__ coef, KFields<T> A, T step, T sdtg, int zero_cur)
 {
     using C = AjCfg<T>;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
+    extern __shared__ unsigned char smem_raw[];
     T *sm = (T *)smem_raw;
     const int ny = p.ny, nz = p.nz;
     // the level tiles of a column run next to each other: their rows share
@@ -1027,20 +1027,38 @@ __global__ void k_adj_project(KParams<T> p, KFields<T> A, T step, int acc)
 
 // Transposed placement of the pressure (the level copies of
 // poisson_fft3d, pressure.cpp:878-892, and mirror_boundaries of PI) + forward
-// FFT along y of the real result.  Block = (spectral row i, level tile).
+// FFT along y of the real result.  Block = (spectral row i, tile of KT level
+// pairs).
+template <typename T>
+__device__ __forceinline__ T adj_pi_placed(const KParams<T> &p, const T *pib, int i, int j, int k)
+{
+    const int nx = p.nx, ny = p.ny, nz = p.nz;
+    T s = T(0);
+    if (i >= 1 && i <= nx - 2 && j >= 1 && j <= ny - 2) {
+        s = pib[gix(ny, nz, i, j, k)];
+        if (i == 1) s += pib[gix(ny, nz, 0, j, k)];
+        if (i == nx - 2) s += pib[gix(ny, nz, nx - 1, j, k)];
+        if (j == 1 || j == ny - 2) {
+            const int jr = j == 1 ? 0 : ny - 1;
+            s += pib[gix(ny, nz, i, jr, k)];
+            if (i == 1) s += pib[gix(ny, nz, 0, jr, k)];
+            if (i == nx - 2) s += pib[gix(ny, nz, nx - 1, jr, k)];
+        }
+    }
+    if (k == 1) s += pib[gix(ny, nz, i, j, 0)];
+    if (k == nz - 2) s += pib[gix(ny, nz, i, j, nz - 1)];
+    return s;
+}
 template <typename T>
 __global__ void k_adj_fft_y_in(KParams<T> p, const T *pib, typename V2<T>::t *spec, FftPlan pj,
                                const typename V2<T>::t *tw, int KT)
 {
     typedef typename V2<T>::t T2;
     extern __shared__ unsigned char smem_raw[];
+    const int ps = fft_ps(KT);
     T2 *a = (T2 *)smem_raw;
-    T2 *b = a + (long)p.nj * KT;
-    const int nx = p.nx, ny = p.ny, nz = p.nz;
-    const int i = blockIdx.y;
-    const int k0 = 1 + blockIdx.x * KT;
-    const int kt = min(KT, nz - 1 - k0);
-    const bool ii = i >= 1 && i <= nx - 2;
+    T2 *b = a + (long)p.nj * ps;
+    const int nz = p.nz, i = blockIdx.y, l0 = blockIdx.x * KT;
     // several rows in flight per thread: the loads of a row do not wait for
     // the previous row's store
 #pragma unroll 4
@@ -1049,30 +1067,13 @@ __global__ void k_adj_fft_y_in(KParams<T> p, const T *pib, typename V2<T>::t *sp
             T2 v;
             v.x = T(0);
             v.y = T(0);
-            if (l < kt) {
-                const int k = k0 + l, j = q;
-                T s = T(0);
-                if (ii && j >= 1 && j <= ny - 2) {
-                    s = pib[gix(ny, nz, i, j, k)];
-                    if (i == 1) s += pib[gix(ny, nz, 0, j, k)];
-                    if (i == nx - 2) s += pib[gix(ny, nz, nx - 1, j, k)];
-                    if (j == 1 || j == ny - 2) {
-                        const int jr = j == 1 ? 0 : ny - 1;
-                        s += pib[gix(ny, nz, i, jr, k)];
-                        if (i == 1) s += pib[gix(ny, nz, 0, jr, k)];
-                        if (i == nx - 2) s += pib[gix(ny, nz, nx - 1, jr, k)];
-                    }
-                }
-                if (k == 1) s += pib[gix(ny, nz, i, j, 0)];
-                if (k == nz - 2) s += pib[gix(ny, nz, i, j, nz - 1)];
-                v.x = s;
-            }
-            a[q * KT + l] = v;
+            const int k = 1 + 2 * (l0 + l);
+            if (k < nz - 1) v.x = adj_pi_placed(p, pib, i, q, k);
+            if (k + 1 < nz - 1) v.y = adj_pi_placed(p, pib, i, q, k + 1);
+            a[q * ps + l] = v;
         }
     __syncthreads();
-    T2 *r = fft_smem<T, T2>(a, b, KT, pj, tw, false, KT);
-    for (int q = threadIdx.y; q < p.nj; q += blockDim.y)
-        for (int l = threadIdx.x; l < kt; l += blockDim.x) spec[((long)i * p.nj + q) * nz + k0 + l] = r[q * KT + l];
+    fft_y_store(p, a, b, spec, pj, tw, KT, i, l0);
 }
 
 // inverse FFT along y and real part: the adjoint of the divergence field
@@ -1083,19 +1084,20 @@ __global__ void k_adj_ifft_y_out(KParams<T> p, const typename V2<T>::t *spec, T 
 {
     typedef typename V2<T>::t T2;
     extern __shared__ unsigned char smem_raw[];
+    const int ps = fft_ps(KT);
     T2 *a = (T2 *)smem_raw;
-    T2 *b = a + (long)p.nj * KT;
-    const int nz = p.nz;
-    const int i = blockIdx.y;
-    const int k0 = 1 + blockIdx.x * KT;
-    const int kt = min(KT, nz - 1 - k0);
-    for (int q = threadIdx.y; q < p.nj; q += blockDim.y)
-        for (int l = threadIdx.x; l < KT; l += blockDim.x)
-            cp_elem(a + q * KT + l, spec + ((long)i * p.nj + q) * nz + k0 + min(l, kt - 1), l < kt);
-    cp_wait_all_sync();
-    T2 *r = fft_smem<T, T2>(a, b, KT, pj, tw, true, KT);
+    T2 *b = a + (long)p.nj * ps;
+    const int nz = p.nz, i = blockIdx.y, l0 = blockIdx.x * KT;
+    const int lt = min(KT, level_pairs(nz) - l0);
+    const T2 *r = fft_y_load(p, a, b, spec, pj, tw, KT, i, l0);
     for (int j = threadIdx.y; j < p.nj; j += blockDim.y)
-        for (int l = threadIdx.x; l < kt; l += blockDim.x) dbar[gix(p.ny, nz, i, j, k0 + l)] = r[j * KT + l].x;
+        for (int l = threadIdx.x; l < lt; l += blockDim.x) {
+            const int k = 1 + 2 * (l0 + l);
+            const T2 v = r[j * ps + l];
+            T *o = dbar + gix(p.ny, nz, i, j, k);
+            o[0] = v.x;
+            if (k + 1 <= nz - 2) o[1] = v.y;
+        }
 }
 
 // Transposed Thomas solve of one wavenumber: M^T z = y / (ni nj), with M the
@@ -1247,14 +1249,14 @@ __global__ void k_spectral_x_adj(KParams<T> p, typename V2<T>::t *spec, FftPlan 
     }
     for (int i = threadIdx.y; i < p.ni; i += blockDim.y)
         for (int l = threadIdx.x; l < nl; l += blockDim.x)
-            cp_elem(a + i * ps + l, spec + ((long)i * p.nj + q) * p.nz + 1 + l, true);
+            cp_elem(a + i * ps + l, spec + spec_at(p, i, q, 1 + l), true);
     cp_wait_all_sync();
-    T2 *r = fft_smem<T, T2>(a, b, nl, pi, tw, false, ps);
+    T2 *r = fft_smem<false, T, T2>(a, b, nl, pi, tw, ps);
     T2 *fr = (r == a) ? b : a;
     const double size2d = (double)(p.ni * p.nj);
     if (sizeof(T) == 8) {
         for (int pp = tid; pp < p.ni; pp += nth) {
-            const long col = (long)pp * p.nj + q;
+            const long col = (long)pp * p.nh + q;
             double *Fw = (double *)(fr + (long)pp * ps) - 1;
             thomas_T_column<T2, double>(r + (long)pp * ps - 1, Fw, p.nz, 2.0 * p.hcoef[col] / p.dx2, 1.0 / size2d, d_r,
                                         d_a, d_c, d_v, col == 0);
@@ -1262,7 +1264,7 @@ __global__ void k_spectral_x_adj(KParams<T> p, typename V2<T>::t *spec, FftPlan 
     } else {
         const float dx2 = (float)p.dx2, inv_s = (float)(1.0 / size2d);
         for (int pp = tid; pp < p.ni; pp += nth) {
-            const long col = (long)pp * p.nj + q;
+            const long col = (long)pp * p.nh + q;
             if (col == 0) continue;  // mean mode: FP64 below
             const float hb = 2.0f * (float)p.hcoef[col] / dx2;
             float *Fw = (float *)(fr + (long)pp * ps) - 1;
@@ -1274,9 +1276,9 @@ __global__ void k_spectral_x_adj(KParams<T> p, typename V2<T>::t *spec, FftPlan 
             pcr_column_T_f64(r - 1, nl, p.hcoef[0], p.dx2, size2d, d_r, d_a, d_c, d_v, pcr_wk);
     }
     __syncthreads();
-    T2 *o = fft_smem<T, T2>(r, fr, nl, pi, tw, true, ps);
+    T2 *o = fft_smem<true, T, T2>(r, fr, nl, pi, tw, ps);
     for (int i = threadIdx.y; i < p.ni; i += blockDim.y)
-        for (int l = threadIdx.x; l < nl; l += blockDim.x) spec[((long)i * p.nj + q) * p.nz + 1 + l] = o[i * ps + l];
+        for (int l = threadIdx.x; l < nl; l += blockDim.x) spec[spec_at(p, i, q, 1 + l)] = o[i * ps + l];
 }
 
 // transposed solves of every wavenumber, TC columns per block staged through
@@ -1290,32 +1292,32 @@ __global__ void k_thomas_adj(KParams<T> p, typename V2<T>::t *spec, int TC)
     const int cs = p.nz | 1;
     T2 *xs = (T2 *)smem_raw;
     T *fs = (T *)(xs + (long)TC * cs);
-    const long ncol = (long)p.ni * p.nj;
-    const long c0 = (long)blockIdx.x * TC;
-    const int nc = (int)min((long)TC, ncol - c0);
-    T2 *g = spec + c0 * p.nz;
-    for (int w = threadIdx.x; w < nc * p.nz; w += blockDim.x) cp_elem(xs + (w / p.nz) * cs + w % p.nz, g + w, true);
-    cp_wait_all_sync();
+    const int ncol = p.ni * p.nh, nl = p.nz - 2;
+    const int c0 = (int)blockIdx.x * TC;
+    const int nc = min(TC, ncol - c0);
+    T2 *g = spec + (long)c0 * p.nzs;
+    columns_in(xs, cs, g, p.nzs, nc, nl);
     const double inv_s = 1.0 / (double)(p.ni * p.nj);
     const bool mean_block = sizeof(T) != 8 && c0 == 0 && p.mean_inv;  // the mean mode, block-wide below
     for (int c = threadIdx.x; c < nc; c += blockDim.x) {
-        const long col = c0 + c;
+        const int col = c0 + c;
+        T2 *x = xs + (long)c * cs - 1;
         if (col == 0 && mean_block) continue;
         if (sizeof(T) == 8 || col == 0) {
             double Floc[PPM_MAXZ];
-            thomas_T_column<T2, double>(xs + (long)c * cs, Floc, p.nz, 2.0 * p.hcoef[col] / p.dx2, inv_s, p.rhou_d,
+            thomas_T_column<T2, double>(x, Floc, p.nz, 2.0 * p.hcoef[col] / p.dx2, inv_s, p.rhou_d,
                                         p.acoef_d, p.ccoef_d, p.vcoef_d, col == 0);
         } else {
-            thomas_T_column<T2, T>(xs + (long)c * cs, fs + (long)c * cs, p.nz, (T)(2.0 * p.hcoef[col] / p.dx2),
+            thomas_T_column<T2, T>(x, fs + (long)c * cs, p.nz, (T)(2.0 * p.hcoef[col] / p.dx2),
                                    (T)inv_s, p.rhou, p.acoef, p.ccoef, p.vcoef, false);
         }
     }
     if (mean_block) {
         __shared__ double mwk[2 * PPM_MAXZ];
-        mean_mode_solve_T(xs, p.nz - 2, p.mean_inv, (double)(p.ni * p.nj), mwk);
+        mean_mode_solve_T(xs - 1, nl, p.mean_inv, (double)(p.ni * p.nj), mwk);
     }
     __syncthreads();
-    for (int w = threadIdx.x; w < nc * p.nz; w += blockDim.x) g[w] = xs[(w / p.nz) * cs + w % p.nz];
+    columns_out(xs, cs, g, p.nzs, nc, nl);
 }
 
 // transposed divergence (divergence3d, pressure.cpp:1340-1381) with its

@@ -48,9 +48,9 @@ __global__ void k_noalloc_tables(int ni, int nj, int nz, double dz, double2 *tw_
                                  double *rhou, double *rhow, double *ac, double *cc, double *vc)
 {
     const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long nh = (long)ni * nj;
-    if (t < nh) {
-        const int p = (int)(t / nj), q = (int)(t % nj);
+    const int nh = spec_nh(nj);
+    if (t < (long)ni * nh) {
+        const int p = (int)(t / nh), q = (int)(t % nh);
         hcoef[t] = cospi(2.0 * p / ni) + cospi(2.0 * q / nj) - 2.0;
     }
     if (t < ni) {
@@ -87,25 +87,6 @@ __global__ void k_noalloc_tables(int ni, int nj, int nz, double dz, double2 *tw_
     }
 }
 
-static FftPlan plan_for(int n)
-{
-    FftPlan P;
-    std::memset(&P, 0, sizeof(P));
-    P.n = n;
-    int m = n;
-    while (m % 4 == 0 && P.nfac < 23) { P.fac[P.nfac++] = 4; m /= 4; }
-    for (int f = 2; m > 1 && P.nfac < 24;) {
-        if (m % f == 0) { P.fac[P.nfac++] = f; m /= f; }
-        else f = (f == 2) ? 3 : f + 2;
-    }
-    int ns = 1;
-    for (int f = 0; f < P.nfac; f++) {
-        P.nslog[f] = (ns & (ns - 1)) == 0 ? __builtin_ctz(ns) : -1;
-        ns *= P.fac[f];
-    }
-    return P;
-}
-
 size_t noalloc_bytes_needed(const ga_config *c)
 {
     const size_t ni = c->periodic_ew_boundaries ? c->nx - 6 : c->nx, nj = c->ny, nz = c->nz;
@@ -138,9 +119,9 @@ static NoallocPlan noalloc_plan(const ga_config *c)
     };
     P.KTy = pow2_tile(P.nj);
     P.KTx = pow2_tile(P.ni);
-    P.smem_y = 2 * (size_t)P.nj * P.KTy * sizeof(double2);
-    P.smem_x = 2 * (size_t)P.ni * P.KTx * sizeof(double2);
-    P.nkt_y = (NZ - 2 + P.KTy - 1) / P.KTy;
+    P.smem_y = fft_bytes(P.nj, P.KTy, sizeof(double2));
+    P.smem_x = fft_bytes(P.ni, P.KTx, sizeof(double2));
+    P.nkt_y = (level_pairs(NZ) + P.KTy - 1) / P.KTy;
     P.nkt_x = (NZ - 2 + P.KTx - 1) / P.KTx;
     const int nl = NZ - 2, m = 8;
     P.ps = nl + ((1 - nl % m) % m + m) % m;
@@ -255,7 +236,7 @@ int solve_pressure_noalloc(const ga_config *c, const ga_columns *cols, double *u
     KParams<double> kp;
     std::memset(&kp, 0, sizeof(kp));
     kp.nx = NX; kp.ny = NY; kp.nz = NZ; kp.n = (long)NX * NY * NZ;
-    kp.ni = ni; kp.nj = nj; kp.ioff = periodic ? 3 : 0; kp.periodic = periodic;
+    kp.ni = ni; kp.nj = nj; kp.nh = spec_nh(nj); kp.nzs = spec_nzs(NZ); kp.ioff = periodic ? 3 : 0; kp.periodic = periodic;
     kp.dt = c->dt;
     kp.one_d_dx = 1.0 / c->dx; kp.one_d_dy = 1.0 / c->dy; kp.one_d_dz = 1.0 / c->dz;
     kp.mu = mu; kp.mw = mw; kp.rhou = rhou; kp.rhow = rhow;
@@ -276,21 +257,21 @@ int solve_pressure_noalloc(const ga_config *c, const ga_columns *cols, double *u
         k_periodic_copy<double><<<(int)((tot + 255) / 256), 256, 0, stream>>>(kp, up, vp, wp, (double *)nullptr);
     }
     // divergence + FFT along y
-    const FftPlan pj = plan_for(nj), pi_plan = plan_for(ni);
+    const FftPlan pj = make_fft_plan(nj), pi_plan = make_fft_plan(ni);
     const dim3 by_y(P.KTy, std::max(1, 256 / P.KTy)), by_x(P.KTx, std::max(1, 256 / P.KTx));
     k_div_fft_y<double><<<dim3(P.nkt_y, ni), by_y, P.smem_y, stream>>>(kp, F, spec, pj, tw_j, step * c->dt, P.KTy);
     // FFT along x + Thomas + inverse FFT along x
     const int nl = NZ - 2;
     if (P.fused) {
         const int bx = std::min(nl, 64);
-        k_spectral_x<double><<<nj, dim3(bx, std::max(1, 256 / bx)), P.smem_spec, stream>>>(kp, spec, pi_plan, tw_i,
+        k_spectral_x<double><<<kp.nh, dim3(bx, std::max(1, 256 / bx)), P.smem_spec, stream>>>(kp, spec, pi_plan, tw_i,
                                                                                          P.ps);
     } else {
         const int TC = kNoallocThomasCols;
-        k_fft_x<double><<<dim3(P.nkt_x, nj), by_x, P.smem_x, stream>>>(kp, spec, pi_plan, tw_i, 0, P.KTx);
-        const long ncol = (long)ni * nj;
+        k_fft_x<double><<<dim3(P.nkt_x, kp.nh), by_x, P.smem_x, stream>>>(kp, spec, pi_plan, tw_i, 0, P.KTx);
+        const long ncol = (long)ni * kp.nh;
         k_thomas<double><<<(int)((ncol + TC - 1) / TC), TC, P.smem_th, stream>>>(kp, spec, TC);
-        k_fft_x<double><<<dim3(P.nkt_x, nj), by_x, P.smem_x, stream>>>(kp, spec, pi_plan, tw_i, 1, P.KTx);
+        k_fft_x<double><<<dim3(P.nkt_x, kp.nh), by_x, P.smem_x, stream>>>(kp, spec, pi_plan, tw_i, 1, P.KTx);
     }
     // inverse FFT along y + PI with the level copies and lateral placement
     k_ifft_y_pi<double><<<dim3(P.nkt_y, ni), by_y, P.smem_y, stream>>>(kp, F, spec, pj, tw_j, P.KTy);

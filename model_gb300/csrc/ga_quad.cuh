@@ -1139,9 +1139,9 @@ __global__ void __cluster_dims__(2, 1, 1) k_spectral_x_pair(KParams<T> p, typena
     // this CTA's levels of every x line
     for (int i = threadIdx.y; i < ni; i += blockDim.y)
         for (int l = threadIdx.x; l < nlr; l += blockDim.x)
-            cp_elem(a + i * ps + l, spec + ((long)i * p.nj + q) * p.nz + 1 + l0 + l, true);
+            cp_elem(a + i * ps + l, spec + spec_at(p, i, q, 1 + l0 + l), true);
     cp_wait_all_sync();
-    float2 *r = fft_smem<float, float2>(a, b, nlr, pi, tw, false, ps);
+    float2 *r = fft_smem<false, float, float2>(a, b, nlr, pi, tw, ps);
     float2 *fr = (r == a) ? b : a;  // free: the Thomas coefficients
     cluster.sync();  // both halves transformed (both CTAs end in the same buffer)
     float2 *pr = cluster.map_shared_rank(r, rank ^ 1);
@@ -1153,14 +1153,13 @@ __global__ void __cluster_dims__(2, 1, 1) k_spectral_x_pair(KParams<T> p, typena
     }
     __syncthreads();
     const double size2d = (double)(ni * p.nj);
-    const int aq = min(q, p.nj - q);
-    const bool q_low = p.low_modes > 0 && aq < p.low_modes;
+    const bool q_low = p.low_modes > 0 && q < p.low_modes;
     {
         const float dx2 = (float)p.dx2, inv_s = (float)(1.0 / size2d);
         for (int pc = tid; pc < np; pc += nth) {
             const int pp = p0 + pc, ap = min(pp, ni - pp);
             if (q_low && ap < p.low_modes) continue;  // FP64 islands below
-            const long col = (long)pp * p.nj + q;
+            const long col = (long)pp * p.nh + q;
             const float hb = 2.0f * (float)p.hcoef[col] / dx2;
             float *Fw = (float *)fr + (long)pc * xs - 1;  // nl floats per column
             thomas_column_fast(X + (long)pc * xs - 1, Fw, p.nz, hb, inv_s, c_r, c_a, c_c, c_v, col == 0);
@@ -1169,7 +1168,7 @@ __global__ void __cluster_dims__(2, 1, 1) k_spectral_x_pair(KParams<T> p, typena
             for (int pc = 0; pc < np; pc++) {
                 const int pp = p0 + pc, ap = min(pp, ni - pp);
                 if (ap >= p.low_modes) continue;
-                const long col = (long)pp * p.nj + q;
+                const long col = (long)pp * p.nh + q;
                 if (col == 0 && p.mean_inv) continue;
                 pcr_column_f64(X + (long)pc * xs - 1, nl, p.hcoef[col], p.dx2, size2d, d_r, d_a, d_c, d_v,
                                col == 0, pcr_wk);
@@ -1188,9 +1187,9 @@ __global__ void __cluster_dims__(2, 1, 1) k_spectral_x_pair(KParams<T> p, typena
         else pr[pp * ps + (l - ol0)] = X[pc * xs + l];
     }
     cluster.sync();  // every column written back
-    float2 *o = fft_smem<float, float2>(r, fr, nlr, pi, tw, true, ps);
+    float2 *o = fft_smem<true, float, float2>(r, fr, nlr, pi, tw, ps);
     for (int i = threadIdx.y; i < ni; i += blockDim.y)
-        for (int l = threadIdx.x; l < nlr; l += blockDim.x) spec[((long)i * p.nj + q) * p.nz + 1 + l0 + l] = o[i * ps + l];
+        for (int l = threadIdx.x; l < nlr; l += blockDim.x) spec[spec_at(p, i, q, 1 + l0 + l)] = o[i * ps + l];
 }
 
 }  // namespace ga
