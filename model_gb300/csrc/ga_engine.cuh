@@ -16,6 +16,7 @@
 #include "ga_engine.h"
 #include "ga_kernels.cuh"
 #include "ga_quad.cuh"
+#include "ga_march.cuh"
 #include "ga_turb.cuh"
 #include "ga_hydro.cuh"
 #include "ga_ice.cuh"
@@ -67,7 +68,7 @@ class Engine : public EngineBase {
     cudaGraphExec_t graph[2] = {nullptr, nullptr};
     bool bar_uniform[6] = {false, false, false, false, false, false};
     bool btab_dirty = true;
-    T *btab = nullptr;
+    T *btab = nullptr, *mtab = nullptr;
     long long graph_launches[2] = {0, 0};
     bool use_graphs = true;
     int status = GA_OK;
@@ -82,6 +83,10 @@ class Engine : public EngineBase {
     // the four-level kernel with the current fields staged into shared memory
     // by the tensor memory accelerator (k_advect_tma), and its candidate
     int adv_tma = 0, adv_tmc = 0;
+    // the marching four-level kernel (k_advect_march), unless GA_ADVECT names
+    // another, and its x chunk (0: march_geom's, or autotuned)
+    int adv_march = 1, adv_li = 0;
+    int nsm = 152;  // SMs of the device
     double *budget_w = nullptr, *budget_part = nullptr;  // FP64 budget weights and partial sums
     T *diff_tend = nullptr;  // explicit diffusion: a second buffer for every prognostic field
     T *diff_buf[9] = {};     // (the one each field's diffused start-of-step values go to)
@@ -275,7 +280,6 @@ class Engine : public EngineBase {
             return;
         }
         {
-            int nsm = 0;
             cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
             overlap = c->ny <= nsm;  // kp.nj = NY blocks in the x solve
             if (const char *ev = std::getenv("GA_OVERLAP")) overlap_rec = overlap = std::strcmp(ev, "0") != 0;
@@ -298,6 +302,7 @@ class Engine : public EngineBase {
         const int nh = spec_nh(nj), nzs = spec_nzs(NZ);
         spec = dalloc<T2>((size_t)ni * nh * nzs);
         btab = dalloc<T>((size_t)BT_COUNT * NZ);
+        mtab = dalloc<T>((size_t)MT_COUNT * NZ);
 
         // ---- scalars (initialize_globals, initializer.cpp:168-179) ----
         const double dx = c->dx, dy = c->dy, dz = c->dz, dt = c->dt;
@@ -548,7 +553,9 @@ class Engine : public EngineBase {
             if (!std::strcmp(ev, "tile")) adv_force = 1;
             else if (!std::strcmp(ev, "quad")) adv_force = 2;
             else if (!std::strcmp(ev, "tma")) adv_force = 3;
+            else if (!std::strcmp(ev, "march")) adv_force = 4;
         }
+        adv_march = adv_force == 0 || adv_force == 4;
         if (const char *ev = std::getenv("GA_ADVECT_TMA")) {  // default staged candidate 0..3
             const int c = std::atoi(ev);
             if (c >= 0 && c < 4) adv_tmc = c;
@@ -577,6 +584,8 @@ class Engine : public EngineBase {
         if constexpr (sizeof(T) == 4) {
             for (auto &tl : kQuadTiles) quad_attr(tl[0], tl[1], optin);
             tma_attr(optin);
+            cudaFuncSetAttribute(k_advect_march<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
+            cudaFuncSetAttribute(k_advect_march<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
         }
         cudaFuncSetAttribute(k_div_fft_y<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
         cudaFuncSetAttribute(k_ifft_y_pi<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
@@ -816,6 +825,13 @@ class Engine : public EngineBase {
             launches++;
         }
         kp.btab = btab;
+        kp.mtab = mtab;
+        if constexpr (sizeof(T) == 4) {
+            if (adv) {
+                k_march_table<<<cdiv(NZ, 128), 128, 0, stream>>>(kp, mtab);
+                launches++;
+            }
+        }
         kp.ubase_adv = adv && !cfg.linear_model;  // the tables hold the full-velocity faces only
         kp.ubase_kes = kes;
     }
@@ -972,6 +988,32 @@ class Engine : public EngineBase {
         return sizeof(T) == 4 && kp.ubase_adv && NZ % 4 == 0 && advect_quad_smem(ti, tj, NZ) <= 200 * 1024;
     }
 
+    // the marching kernel applies: FP32, basic state a function of height,
+    // whole quads of levels
+    bool use_march() const { return sizeof(T) == 4 && adv_march && kp.ubase_adv && NZ % 4 == 0; }
+    // a four-level advection kernel runs that also takes the mirror copies,
+    // and snow and ice in the moisture launch
+    bool adv_takes_mirror() const { return use_march() || (adv_quad && quad_ok(adv_qi, adv_qj)); }
+    bool adv_takes_ice() const
+    {
+        return use_march() || (adv_quad && quad_ok(adv_qi, adv_qj) && !(adv_tma && tma_ok(adv_tmc)));
+    }
+    void launch_march(T step, T sdtg, int what)
+    {
+        if constexpr (sizeof(T) == 4) {
+            int nj = 0;
+            const unsigned long long jobs = march_jobs(what, qmask != nullptr, &nj);
+            const MarchGeom g = march_geom(NX, NY, NZ, nj, nsm, adv_li);
+            const int by_job = march_by_job(N);
+            const dim3 grid = by_job ? dim3(g.njt, g.nit, nj) : dim3(nj, g.nit, g.njt);
+            const size_t sm = march_smem(g.tj, NZ);
+            if (by_job)
+                k_advect_march<2><<<grid, AM_THREADS, sm, stream>>>(kp, fields(), g, jobs, by_job, step, sdtg, what);
+            else
+                k_advect_march<3><<<grid, AM_THREADS, sm, stream>>>(kp, fields(), g, jobs, by_job, step, sdtg, what);
+        }
+    }
+
     // apply_explicit_diffusion (damping.cpp:1125-1146) on the start-of-step slot
     void diffuse(double step)
     {
@@ -1059,7 +1101,9 @@ class Engine : public EngineBase {
     {
         const double sdtg = step * cfg.dt * 9.8 * 0.5;  // step*dt*grav*0.5, advection.cpp:330
         ProfScope ps(this, PC_ADVECT, 1);
-        if (adv_quad && adv_tma && tma_ok(adv_tmc)) {
+        if (use_march()) {
+            launch_march((T)step, (T)sdtg, what);
+        } else if (adv_quad && adv_tma && tma_ok(adv_tmc)) {
             launch_advect_tma_cand(adv_tmc, (T)step, (T)sdtg, what);
         } else if (adv_quad && quad_ok(adv_qi, adv_qj)) {
             const T st = (T)step, sg = (T)sdtg;
@@ -1501,7 +1545,7 @@ class Engine : public EngineBase {
                 hyd_solve(st);
                 hyd_project(st);
                 if (ice) {
-                    const bool quad = adv_quad && quad_ok(adv_qi, adv_qj) && !(adv_tma && tma_ok(adv_tmc));
+                    const bool quad = adv_takes_ice();
                     if (kp.rf == 1) ice_fall_euler(IF_RAIN | IF_SNOW | IF_ICE);
                     if (quad) {
                         advect(st, ADV_Q | ADV_ICE | ADV_ZERO);
@@ -1526,8 +1570,8 @@ class Engine : public EngineBase {
                 // the Rutledge fall speeds read the pressure of this stage's
                 // solve, so the moisture advection follows it; the four-level
                 // kernel (FP32) advects snow and ice in the same launch
-                const bool quad = adv_quad && quad_ok(adv_qi, adv_qj) && !(adv_tma && tma_ok(adv_tmc));
-                const bool fuse = !kp.periodic && quad;
+                const bool quad = adv_takes_ice();
+                const bool fuse = !kp.periodic && adv_takes_mirror();
                 const bool side = overlap && !prof;  // theta beside the solve
                 advect(st, ADV_UV | ADV_WB | (side ? 0 : ADV_TH) | (fuse ? ADV_MIRROR : 0));
                 if (turbulent) turb_apply(side ? TA_VEL : TA_VEL | TA_TH, st);
@@ -1563,7 +1607,7 @@ class Engine : public EngineBase {
             }
             // the four-level advection launch also makes the mirror copies of
             // the pressure solve (they touch no point the advection writes)
-            const bool fuse_mirror = !kp.periodic && adv_quad && quad_ok(adv_qi, adv_qj);
+            const bool fuse_mirror = !kp.periodic && adv_takes_mirror();
             // with turbulence the stage's tendencies come after the advection
             // and before zero_moisture (driver_serial.cpp:205-230), which the
             // post-processing pass then applies; they touch no point that the
@@ -1736,8 +1780,22 @@ class Engine : public EngineBase {
         const int what = ADV_UV | ADV_WB | ADV_TH | (kp.moist ? (ADV_Q | ADV_ZERO) : 0);
         std::string info;
         char line[160];
-        // advection tile
-        {
+        if (use_march()) {  // its x chunk: the launch rule's, or a fixed length
+            float best = 1e30f;
+            int bl = 0;
+            for (int li : {0, 4, 6, 8, 16}) {
+                adv_li = li;
+                const float t = timeit([&] { advect(1. / 3., what); });
+                if (t < best) { best = t; bl = li; }
+            }
+            adv_li = bl;
+            int nj = 0;
+            march_jobs(what, false, &nj);
+            const MarchGeom g = march_geom(NX, NY, NZ, nj, nsm, bl);
+            std::snprintf(line, sizeof line, "advect tile %dx%d, marching, four levels per thread (%.4f ms); ", g.li,
+                          g.tj, best);
+            info += line;
+        } else {  // advection tile
             float best = 1e30f;
             int bi = adv_ti, bj = adv_tj, bq = 0, qi = adv_qi, qj = adv_qj, qb = adv_qb, br = adv_rows;
             int bt = 0, tc = adv_tmc;

@@ -25,6 +25,7 @@ struct MemberAux {
     typename V2<T>::t *spec, *tw_i, *tw_j;
     FftPlan plan_i, plan_j;
     int KTy, psx;
+    MarchGeom march;
 };
 
 enum { EK_ADV = 0, EK_MIRROR, EK_DIVY, EK_SX, EK_IFFTY, EK_POST, EK_KES, EK_FX, EK_TH, EK_COUNT };
@@ -56,25 +57,26 @@ __global__ void __launch_bounds__(256) kb_advect(const KParams<T> *P, const KFie
     }
 }
 
-// FP32 members with whole level quads: the four-level advection and post
-template <typename T, int TI, int TJ, int MB>
-__global__ void __launch_bounds__(AQ_THREADS, MB) kb_advect_quad(const KParams<T> *__restrict__ P,
+// FP32 members with whole level quads: the marching advection and the
+// four-level post.  A member's blocks go job by job (march_by_job), its tile
+// geometry is in its MemberAux.
+template <typename T>
+__global__ void __launch_bounds__(AM_THREADS, 2) kb_advect_march(const KParams<T> *__restrict__ P,
                                                                const KFields<T> *__restrict__ F,
-                                                               const long *__restrict__ pre, int nmem, double step,
-                                                               int what)
+                                                               const MemberAux<T> *__restrict__ A,
+                                                               const long *__restrict__ pre, int nmem,
+                                                               unsigned long long jobs, double step, int what)
 {
     static_assert(sizeof(T) == 4, "four-level kernels are FP32");
     const long total = pre[nmem];
     for (long vb = blockIdx.x; vb < total; vb += gridDim.x) {
         const int m = find_member(pre, nmem, vb);
         const KParams<T> &p = P[m];
-        const long lb = vb - pre[m];
-        const int gx = (p.nx - 6 + TI - 1) / TI;
+        const MarchGeom g = A[m].march;
+        const int lb = (int)(vb - pre[m]), r = lb / g.njt, jb = r / g.nit;
         const double sdtg = step * p.dt_d * 9.8 * 0.5;  // step*dt*grav*0.5, advection.cpp:330
-        // the row form spills in this kernel at either register budget;
-        // masking ADV_ROWS lets the compiler drop it
-        advect_quad_body<TI, TJ>(p, F[m], (int)(lb % gx), (int)(lb / gx), (T)step, (T)sdtg, what & ~ADV_ROWS);
-        __syncthreads();
+        march_body(p, F[m], g, (int)((jobs >> (4 * jb)) & 15ull), r - jb * g.nit, lb - r * g.njt, (T)step, (T)sdtg,
+                   what);
     }
 }
 template <typename T>
@@ -218,25 +220,29 @@ class Ensemble : public EnsembleBase {
     int dev = 0;
     int adv_ti = ADV_TI, adv_tj = ADV_TJ;  // advection tile of every member (autotuned)
     // FP32 members with whole level quads run the four-level post, and the
-    // four-level advection (tile adv_qi x adv_qj) while every basic state is
-    // a function of height and adv_quad is set (autotuned)
-    bool quad = false, adv_quad = true;
-    int adv_qi = 4, adv_qj = 8, adv_qb = 3;  // quad tile, blocks per SM of its register budget
+    // marching advection while every basic state is a function of height and
+    // adv_march is set (autotuned); adv_li: its x chunk (0: march_geom's)
+    bool quad = false, adv_march = true;
+    int adv_li = 16;
     int sx_threads = 256;  // threads of a fused spectral-x block (autotuned)
     // the x solve: fused kernel (0) or x FFT, Thomas, inverse x FFT (1), the
     // level tile of the x FFTs and the columns of a Thomas block (autotuned)
     int sx_unfused = 0, KTx = 8, TC = 64;
     bool fused_ok = true;  // every member fits the fused x kernel
     int nsm = 0;
-    bool adv_quad_now = false;  // the choice build_prefixes made (prefixes and launches agree)
-    bool quad_applies() const
+    bool march_now = false;  // the choice build_prefixes made (prefixes and launches agree)
+    bool march_applies() const
     {
-        if (!quad || !adv_quad) return false;
+        if (!quad || !adv_march) return false;
         for (auto *e : mem)
-            if (!e->quad_ok(adv_qi, adv_qj)) return false;
+            if (!e->kp.ubase_adv) return false;
         return true;
     }
-    bool use_adv_quad() const { return adv_quad_now; }
+    // the step advects everything in one launch: u, v, w's buoyancy, theta
+    // and the moisture
+    int step_jobs() const { return moist ? 7 : 4; }
+    // a member's tile: chunks of up to 16 columns (many members fill the GPU)
+    MarchGeom member_march(const Engine<T> &e) const { return march_geom(e.NX, e.NY, e.NZ, step_jobs(), nsm, adv_li); }
 
     Ensemble(const ga_config *cfgs, const ga_columns *cols, int n, int *rc)
     {
@@ -285,16 +291,7 @@ class Ensemble : public EnsembleBase {
         if constexpr (sizeof(T) == 4) {
             quad = true;
             for (auto *e : mem) quad = quad && e->NZ % 4 == 0;
-            cudaFuncSetAttribute(kb_advect_quad<T, 4, 4, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
-            cudaFuncSetAttribute(kb_advect_quad<T, 4, 4, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
-            cudaFuncSetAttribute(kb_advect_quad<T, 4, 8, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
-            cudaFuncSetAttribute(kb_advect_quad<T, 4, 8, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
-            cudaFuncSetAttribute(kb_advect_quad<T, 8, 4, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
-            cudaFuncSetAttribute(kb_advect_quad<T, 8, 4, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
-            cudaFuncSetAttribute(kb_advect_quad<T, 2, 8, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
-            cudaFuncSetAttribute(kb_advect_quad<T, 2, 8, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
-            cudaFuncSetAttribute(kb_advect_quad<T, 8, 8, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
-            cudaFuncSetAttribute(kb_advect_quad<T, 8, 8, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
+            cudaFuncSetAttribute(kb_advect_march<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
         }
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
         build_prefixes();
@@ -317,29 +314,10 @@ class Ensemble : public EnsembleBase {
         if (stream) cudaStreamDestroy(stream);
     }
 
-    // the batched four-level advection of tile TI x TJ in the chosen register budget
-    template <int TI, int TJ>
-    const void *quad_fn() const
-    {
-        if (adv_qb == 4) return (const void *)kb_advect_quad<T, TI, TJ, 4>;
-        return (const void *)kb_advect_quad<T, TI, TJ, 3>;
-    }
-    template <int TI, int TJ>
-    void launch_quad(dim3 g, size_t sm, const long *pr, const KFields<T> *F, double st, int what)
-    {
-        if (adv_qb == 4) kb_advect_quad<T, TI, TJ, 4><<<g, AQ_THREADS, sm, stream>>>(d_p, F, pr, nmem, st, what);
-        else kb_advect_quad<T, TI, TJ, 3><<<g, AQ_THREADS, sm, stream>>>(d_p, F, pr, nmem, st, what);
-    }
     const void *advect_fn() const
     {
         if constexpr (sizeof(T) == 4) {
-            if (use_adv_quad()) {
-                if (adv_qi == 4 && adv_qj == 4) return quad_fn<4, 4>();
-                if (adv_qi == 8 && adv_qj == 4) return quad_fn<8, 4>();
-                if (adv_qi == 2) return quad_fn<2, 8>();
-                if (adv_qi == 8) return quad_fn<8, 8>();
-                return quad_fn<4, 8>();
-            }
+            if (march_now) return (const void *)kb_advect_march<T>;
         }
         if (adv_ti == 2) return (const void *)kb_advect<T, 2, 4>;
         if (adv_tj == 2) return (const void *)kb_advect<T, 4, 2>;
@@ -353,12 +331,10 @@ class Ensemble : public EnsembleBase {
         const size_t sm = smem[EK_ADV];
         const long *pr = d_pre[EK_ADV];
         if constexpr (sizeof(T) == 4) {
-            if (use_adv_quad()) {
-                if (adv_qi == 4 && adv_qj == 4) launch_quad<4, 4>(g, sm, pr, F, st, what);
-                else if (adv_qi == 8 && adv_qj == 4) launch_quad<8, 4>(g, sm, pr, F, st, what);
-                else if (adv_qi == 2) launch_quad<2, 8>(g, sm, pr, F, st, what);
-                else if (adv_qi == 8) launch_quad<8, 8>(g, sm, pr, F, st, what);
-                else launch_quad<4, 8>(g, sm, pr, F, st, what);
+            if (march_now) {
+                int nj = 0;
+                const unsigned long long jobs = march_jobs(what, false, &nj);
+                kb_advect_march<T><<<g, AM_THREADS, sm, stream>>>(d_p, F, d_aux, pr, nmem, jobs, st, what);
                 return;
             }
         }
@@ -407,7 +383,7 @@ class Ensemble : public EnsembleBase {
     void build_prefixes()
     {
         const int n = nmem;
-        adv_quad_now = quad_applies();
+        march_now = march_applies();
         for (int k = 0; k < EK_COUNT; k++) {
             std::vector<long> pre(n + 1, 0);
             size_t sm = 0;
@@ -416,9 +392,10 @@ class Ensemble : public EnsembleBase {
                 long c = 0;
                 switch (k) {
                 case EK_ADV:
-                    if (use_adv_quad()) {
-                        c = (long)cdiv(e.NX - 6, adv_qi) * cdiv(e.NY - 6, adv_qj);
-                        sm = std::max(sm, advect_quad_smem(adv_qi, adv_qj, e.NZ));
+                    if (march_now) {
+                        const MarchGeom g = member_march(e);
+                        c = (long)step_jobs() * g.nit * g.njt;
+                        sm = std::max(sm, march_smem(g.tj, e.NZ));
                     } else {
                         c = (long)cdiv(e.NX - 6, adv_ti) * cdiv(e.NY - 6, adv_tj);
                         sm = std::max(sm, advect_tile_smem(adv_ti, adv_tj, e.NZ, sizeof(T)));
@@ -459,7 +436,7 @@ class Ensemble : public EnsembleBase {
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, fn, threads, sm);
             return std::max(1, b) * nsm;
         };
-        grid[EK_ADV] = occ(advect_fn(), 256, smem[EK_ADV]);
+        grid[EK_ADV] = occ(advect_fn(), march_now ? AM_THREADS : 256, smem[EK_ADV]);
         grid[EK_MIRROR] = occ((const void *)kb_mirror<T>, 256, 0);
         grid[EK_DIVY] = occ((const void *)kb_div_fft_y<T>, 256, smem[EK_DIVY]);
         grid[EK_SX] = occ((const void *)kb_spectral_x<T>, 256, smem[EK_SX]);
@@ -522,44 +499,38 @@ class Ensemble : public EnsembleBase {
         char line[160];
         {
             float best = 1e30f;
-            int bi = adv_ti, bj = adv_tj, qi = adv_qi, qj = adv_qj, qb = adv_qb;
-            bool bq = false;
-            adv_quad = false;
-            for (auto &tl : Engine<T>::kAdvTiles) {
-                bool fits = true;
-                for (auto *e : mem) fits = fits && advect_tile_smem(tl[0], tl[1], e->NZ, sizeof(T)) <= 200 * 1024;
-                if (!fits) continue;
-                adv_ti = tl[0];
-                adv_tj = tl[1];
-                build_prefixes();
-                const float t = timeit([&] { launch_advect(F, 1. / 3., what); });
-                if (t < best) { best = t; bi = tl[0]; bj = tl[1]; }
-            }
-            if (quad) {
-                adv_quad = true;
-                for (auto &tl : Engine<T>::kQuadTiles) {
-                    for (int mb = 3; mb <= 4; mb++) {
-                        adv_qi = tl[0];
-                        adv_qj = tl[1];
-                        adv_qb = mb;
-                        if (!quad_applies()) continue;
-                        build_prefixes();
-                        const float t = timeit([&] { launch_advect(F, 1. / 3., what); });
-                        if (t < best) { best = t; bq = true; qi = tl[0]; qj = tl[1]; qb = mb; }
-                    }
+            if (march_applies()) {  // the marching kernel, its x chunk
+                int bl = adv_li;
+                auto set_li = [&](int li) {
+                    adv_li = li;
+                    tables_dirty = true;
+                    refresh_tables();
+                };
+                for (int li : {4, 8, 16, 32}) {
+                    set_li(li);
+                    const float t = timeit([&] { launch_advect(d_f[rot], 1. / 3., what); });
+                    if (t < best) { best = t; bl = li; }
                 }
+                set_li(bl);
+                std::snprintf(line, sizeof line, "advect tile %d x columns, marching, four levels per thread (%.3f ms); ",
+                              bl, best);
+            } else {
+                int bi = adv_ti, bj = adv_tj;
+                for (auto &tl : Engine<T>::kAdvTiles) {
+                    bool fits = true;
+                    for (auto *e : mem) fits = fits && advect_tile_smem(tl[0], tl[1], e->NZ, sizeof(T)) <= 200 * 1024;
+                    if (!fits) continue;
+                    adv_ti = tl[0];
+                    adv_tj = tl[1];
+                    build_prefixes();
+                    const float t = timeit([&] { launch_advect(F, 1. / 3., what); });
+                    if (t < best) { best = t; bi = tl[0]; bj = tl[1]; }
+                }
+                adv_ti = bi;
+                adv_tj = bj;
+                build_prefixes();
+                std::snprintf(line, sizeof line, "advect tile %dx%d (%.3f ms); ", bi, bj, best);
             }
-            adv_ti = bi;
-            adv_tj = bj;
-            adv_quad = bq;
-            adv_qi = qi;
-            adv_qj = qj;
-            adv_qb = qb;
-            build_prefixes();
-            if (bq)
-                std::snprintf(line, sizeof line, "advect tile %dx%d, four levels per thread, %d blocks/SM (%.3f ms); ", qi,
-                              qj, qb, best);
-            else std::snprintf(line, sizeof line, "advect tile %dx%d (%.3f ms); ", bi, bj, best);
             info += line;
         }
         {
@@ -676,6 +647,7 @@ class Ensemble : public EnsembleBase {
             ha[m].spec = e.spec; ha[m].tw_i = e.tw_i; ha[m].tw_j = e.tw_j;
             ha[m].plan_i = e.plan_i; ha[m].plan_j = e.plan_j;
             ha[m].KTy = e.KTy; ha[m].psx = e.psx;
+            ha[m].march = member_march(e);
         }
         cudaMemcpy(d_p, hp.data(), sizeof(KParams<T>) * nmem, cudaMemcpyHostToDevice);
         cudaMemcpy(d_f[0], f0.data(), sizeof(KFields<T>) * nmem, cudaMemcpyHostToDevice);

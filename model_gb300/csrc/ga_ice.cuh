@@ -169,14 +169,12 @@ __global__ void __launch_bounds__(128) k_advect_ice(KParams<T> p, KFields<T> F, 
     const T *fall[2] = {F.sts, F.its};
     for (int n = 0; n < 2; n++) {
         const T *q = F.cur[fld[n]];
-        T tend = -p.dtx * (s_east(p, F, q, (const T *)nullptr, i, j, k) -
-                           s_east(p, F, q, (const T *)nullptr, i - 1, j, k)) -
-                 p.dty * (s_north(p, F, q, (const T *)nullptr, i, j, k) -
-                          s_north(p, F, q, (const T *)nullptr, i, j - 1, k)) -
-                 DTZ * (p.rhow[k + 1] * fall_top(p, F, q, fall[n], i, j, k) -
-                        p.rhow[k] * fall_top(p, F, q, fall[n], i, j, k - 1)) *
-                     p.one_d_rhou[k];
-        F.P[fld[n]][c] = LD(F.M[fld[n]], c) + step * tend;
+        const T tend = flux_div(
+            p.dtx, s_east(p, F, q, (const T *)nullptr, i, j, k) - s_east(p, F, q, (const T *)nullptr, i - 1, j, k),
+            p.dty, s_north(p, F, q, (const T *)nullptr, i, j, k) - s_north(p, F, q, (const T *)nullptr, i, j - 1, k),
+            DTZ, p.rhow[k + 1], fall_top(p, F, q, fall[n], i, j, k), p.rhow[k],
+            fall_top(p, F, q, fall[n], i, j, k - 1), p.one_d_rhou[k]);
+        F.P[fld[n]][c] = fma_(step, tend, LD(F.M[fld[n]], c));
     }
 }
 

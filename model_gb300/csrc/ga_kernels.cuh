@@ -55,6 +55,7 @@ struct KParams {
     int ubase_adv;  // UBAR, VBAR, WBAR, THBAR, QBAR depend on k only
     int ubase_kes;  // THBAR, QBAR, PBAR depend on k only
     const T *btab;
+    const T *mtab;  // rows of the marching advection kernel (MT_*), FP32
     // the linearised model (ISLINEAR): perturbation faces advected by the
     // basic-state velocity alone; stale_signs: its driver's theta and vapour
     // faces take upwind signs of zero (the sign arrays it never computes)
@@ -122,21 +123,77 @@ template <typename T> struct W {
     static constexpr T c1_60 = T(1.0 / 60.0);
 };
 
-// INTERP_5TH_EAST (fluxes.cpp:110-122, 155-180): stencil a(-2)..a(+3)
+// Products and sums of the advection, written out.  FP64: the reference's
+// operations one by one (ga_f64.cu is compiled without contraction).  FP32:
+// fixed fused multiply-adds, so that every advection kernel, whatever the
+// compiler makes of the code around an expression (packed lanes, selects),
+// rounds it the same way.
+__device__ __forceinline__ double fma_(double a, double b, double c) { return a * b + c; }
+__device__ __forceinline__ float fma_(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double mul_(double a, double b) { return a * b; }
+__device__ __forceinline__ float mul_(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double add_(double a, double b) { return a + b; }
+__device__ __forceinline__ float add_(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ double sub_(double a, double b) { return a - b; }
+__device__ __forceinline__ float sub_(float a, float b) { return __fsub_rn(a, b); }
+
+// INTERP_5TH_EAST (fluxes.cpp:110-122, 155-180): stencil a(-2)..a(+3); cs is
+// the upwind sign times 1/60
+template <typename T>
+__device__ __forceinline__ T face5_cs(T am2, T am1, T a0, T a1, T a2, T a3, T cs)
+{
+    const T c6 = fma_(W<T>::c1_60, add_(a3, am2),
+                      fma_(-W<T>::c2_15, add_(a2, am1), mul_(W<T>::c37_60, add_(a1, a0))));
+    const T u5 = fma_(T(-10.0), sub_(a1, a0), fma_(T(5.0), sub_(a2, am1), -sub_(a3, am2)));
+    return fma_(cs, u5, c6);
+}
 template <typename T>
 __device__ __forceinline__ T face5(T am2, T am1, T a0, T a1, T a2, T a3, T sign)
 {
-    T c6 = W<T>::c37_60 * (a1 + a0) - W<T>::c2_15 * (a2 + am1) + W<T>::c1_60 * (a3 + am2);
-    T u5 = -(a3 - am2) + T(5.0) * (a2 - am1) - T(10.0) * (a1 - a0);
-    return c6 + W<T>::c1_60 * sign * u5;
+    return face5_cs(am2, am1, a0, a1, a2, a3, mul_(W<T>::c1_60, sign));
 }
-// INTERP_3RD_TOP (fluxes.cpp:131-136, 185-199): stencil a(-1)..a(+2)
+// INTERP_3RD_TOP (fluxes.cpp:131-136, 185-199): stencil a(-1)..a(+2); cs is
+// the upwind sign times 1/12
+template <typename T>
+__device__ __forceinline__ T face3_cs(T am1, T a0, T a1, T a2, T cs)
+{
+    const T c4 = fma_(-W<T>::c1_12, add_(a2, am1), mul_(W<T>::c7_12, add_(a1, a0)));
+    const T u3 = fma_(T(-3.0), sub_(a1, a0), sub_(a2, am1));
+    return fma_(cs, u3, c4);
+}
 template <typename T>
 __device__ __forceinline__ T face3(T am1, T a0, T a1, T a2, T sign)
 {
-    T c4 = W<T>::c7_12 * (a1 + a0) - W<T>::c1_12 * (a2 + am1);
-    T u3 = (a2 - am1) - T(3.0) * (a1 - a0);
-    return c4 + W<T>::c1_12 * sign * u3;
+    return face3_cs(am1, a0, a1, a2, mul_(W<T>::c1_12, sign));
+}
+// a flux a*b + c*d
+template <typename T>
+__device__ __forceinline__ T flux2(T a, T b, T c, T d)
+{
+    return fma_(a, b, mul_(c, d));
+}
+// flux divergence of a cell (advection.cpp:73-122, :152-213): east minus west
+// de, north minus south dn, the top faces th and tl with their densities
+template <typename T>
+__device__ __forceinline__ T flux_div(T dtx, T de, T dty, T dn, T DTZ, T rhi, T th, T rlo, T tl, T odr)
+{
+    const T v = fma_(-rlo, tl, mul_(rhi, th));
+    return fma_(-mul_(DTZ, v), odr, fma_(-dty, dn, mul_(-dtx, de)));
+}
+// less the vertical advection of the base profile (Z_ADVECT_BASE,
+// advection.cpp:16-18): w at k+1 and k, the profile's steps above and below
+template <typename T>
+__device__ __forceinline__ T sub_base(T t, T DTZ, T rhi, T wh, T bh, T rlo, T wl, T bl, T odr)
+{
+    const T z = fma_(mul_(rhi, wh), bh, mul_(mul_(rlo, wl), bl));
+    return fma_(-DTZ, mul_(mul_(T(0.50), z), odr), t);
+}
+// buoyancy of a point (advection.cpp:46-60): theta'/tbv, and when moist with
+// vapour, cloud water and rain
+template <typename T>
+__device__ __forceinline__ T buoy_moist(T th, T tbv, T qv, T qc, T qr)
+{
+    return sub_(sub_(fma_(T(0.61), qv, th / tbv), qc), qr);
 }
 
 template <typename T>
@@ -200,7 +257,7 @@ __device__ T u_east(const KParams<T> &p, const KFields<T> &F, int i, int j, int 
     const T at = adv_vel(p, uba, ua);
     T ue = f5i(U, p, i, j, k, sgn(at));
     T ube = f5i(UB, p, i, j, k, sgn(ua));
-    return ua * ube + at * ue;
+    return flux2(ua, ube, at, ue);
 }
 template <typename T>
 __device__ T u_north(const KParams<T> &p, const KFields<T> &F, int i, int j, int k)
@@ -212,7 +269,7 @@ __device__ T u_north(const KParams<T> &p, const KFields<T> &F, int i, int j, int
     const T at = adv_vel(p, vba, va);
     T un = f5j(U, p, i, j, k, sgn(at));
     T ubn = f5j(UB, p, i, j, k, sgn(va));
-    return va * ubn + at * un;
+    return flux2(va, ubn, at, un);
 }
 template <typename T>
 __device__ T u_top(const KParams<T> &p, const KFields<T> &F, int i, int j, int k)
@@ -230,7 +287,7 @@ __device__ T u_top(const KParams<T> &p, const KFields<T> &F, int i, int j, int k
         ut = f3k(U, p, i, j, k, sgn(adv_vel(p, wba, wa)));
         ubt = f3k(UB, p, i, j, k, sgn(wa));
     }
-    return wa * ubt + adv_vel(p, wba, wa) * ut;
+    return flux2(wa, ubt, adv_vel(p, wba, wa), ut);
 }
 template <typename T>
 __device__ T v_east(const KParams<T> &p, const KFields<T> &F, int i, int j, int k)
@@ -242,7 +299,7 @@ __device__ T v_east(const KParams<T> &p, const KFields<T> &F, int i, int j, int 
     const T at = adv_vel(p, uba, ua);
     T ve = f5i(V, p, i, j, k, sgn(at));
     T vbe = f5i(VB, p, i, j, k, sgn(ua));
-    return ua * vbe + at * ve;
+    return flux2(ua, vbe, at, ve);
 }
 template <typename T>
 __device__ T v_north(const KParams<T> &p, const KFields<T> &F, int i, int j, int k)
@@ -254,7 +311,7 @@ __device__ T v_north(const KParams<T> &p, const KFields<T> &F, int i, int j, int
     const T at = adv_vel(p, vba, va);
     T vn = f5j(V, p, i, j, k, sgn(at));
     T vbn = f5j(VB, p, i, j, k, sgn(va));
-    return va * vbn + at * vn;
+    return flux2(va, vbn, at, vn);
 }
 template <typename T>
 __device__ T v_top(const KParams<T> &p, const KFields<T> &F, int i, int j, int k)
@@ -272,7 +329,7 @@ __device__ T v_top(const KParams<T> &p, const KFields<T> &F, int i, int j, int k
         vt = f3k(V, p, i, j, k, sgn(adv_vel(p, wba, wa)));
         vbt = f3k(VB, p, i, j, k, sgn(wa));
     }
-    return wa * vbt + adv_vel(p, wba, wa) * vt;
+    return flux2(wa, vbt, adv_vel(p, wba, wa), vt);
 }
 
 // ---------------------------------------------------------------------------
@@ -292,7 +349,7 @@ __device__ T s_east(const KParams<T> &p, const KFields<T> &F, const T *s, const 
     T se = f5i(s, p, i, j, k, z ? T(0) : sgn(ut));
     if (!sb) return ut * se;
     T be = f5i(sb, p, i, j, k, z ? T(0) : sgn(u1));
-    return u1 * be + ut * se;
+    return flux2(u1, be, ut, se);
 }
 template <typename T>
 __device__ T s_north(const KParams<T> &p, const KFields<T> &F, const T *s, const T *sb, int i, int j, int k)
@@ -304,7 +361,7 @@ __device__ T s_north(const KParams<T> &p, const KFields<T> &F, const T *s, const
     T sn = f5j(s, p, i, j, k, z ? T(0) : sgn(vt));
     if (!sb) return vt * sn;
     T bn = f5j(sb, p, i, j, k, z ? T(0) : sgn(v1));
-    return v1 * bn + vt * sn;
+    return flux2(v1, bn, vt, sn);
 }
 template <typename T>
 __device__ T s_top(const KParams<T> &p, const KFields<T> &F, const T *s, const T *sb, int i, int j, int k)
@@ -323,7 +380,7 @@ __device__ T s_top(const KParams<T> &p, const KFields<T> &F, const T *s, const T
         if (sb) bt = f3k(sb, p, i, j, k, z ? T(0) : sgn(w1));
     }
     if (!sb) return wt * st;
-    return w1 * bt + wt * st;
+    return flux2(w1, bt, wt, st);
 }
 
 // rain fall speed of one point: calculate_rain_fall_speed_kessler
@@ -378,17 +435,13 @@ __device__ T s_tend(const KParams<T> &p, const KFields<T> &F, const T *s, const 
                     int i, int j, int k)
 {
     const T DTZ = p.dtz * p.mu[k];
-    T t = -p.dtx * (s_east(p, F, s, sb, i, j, k) - s_east(p, F, s, sb, i - 1, j, k)) -
-          p.dty * (s_north(p, F, s, sb, i, j, k) - s_north(p, F, s, sb, i, j - 1, k)) -
-          DTZ * (p.rhow[k + 1] * s_top(p, F, s, sb, i, j, k) - p.rhow[k] * s_top(p, F, s, sb, i, j, k - 1)) *
-              p.one_d_rhou[k];
+    T t = flux_div(p.dtx, s_east(p, F, s, sb, i, j, k) - s_east(p, F, s, sb, i - 1, j, k), p.dty,
+                   s_north(p, F, s, sb, i, j, k) - s_north(p, F, s, sb, i, j - 1, k), DTZ, p.rhow[k + 1],
+                   s_top(p, F, s, sb, i, j, k), p.rhow[k], s_top(p, F, s, sb, i, j, k - 1), p.one_d_rhou[k]);
     if (base) {
         const T *Wc = F.cur[FW];
-        T zab = T(0.50) *
-                (p.rhow[k + 1] * LD(Wc, gix(p.ny, p.nz, i, j, k + 1)) * (base[k + 1] - base[k]) +
-                 p.rhow[k] * LD(Wc, gix(p.ny, p.nz, i, j, k)) * (base[k] - base[k - 1])) *
-                p.one_d_rhou[k];
-        t = t - DTZ * zab;
+        t = sub_base(t, DTZ, p.rhow[k + 1], LD(Wc, gix(p.ny, p.nz, i, j, k + 1)), base[k + 1] - base[k], p.rhow[k],
+                     LD(Wc, gix(p.ny, p.nz, i, j, k)), base[k] - base[k - 1], p.one_d_rhou[k]);
     }
     return t;
 }
@@ -423,19 +476,17 @@ __global__ void __launch_bounds__(128) k_advect(KParams<T> p, KFields<T> F, T st
         const T *U = F.cur[FU], *V = F.cur[FV];
         const long sy = p.nz, sx = (long)p.ny * p.nz;
         T ov_u = T(0.25) * (LD(V, c) + LD(V, c + sy) + LD(V, c - sx) + LD(V, c - sx + sy));
-        T ut = -p.dtx * (u_east(p, F, i, j, k) - u_east(p, F, i - 1, j, k)) -
-               p.dty * (u_north(p, F, i, j, k) - u_north(p, F, i, j - 1, k)) -
-               DTZ * (p.rhow[k + 1] * u_top(p, F, i, j, k) - p.rhow[k] * u_top(p, F, i, j, k - 1)) *
-                   p.one_d_rhou[k] +
-               p.dt * p.f[j] * ov_u;
-        F.P[FU][c] = LD(F.M[FU], c) + step * ut;
+        T ut = flux_div(p.dtx, u_east(p, F, i, j, k) - u_east(p, F, i - 1, j, k), p.dty,
+                        u_north(p, F, i, j, k) - u_north(p, F, i, j - 1, k), DTZ, p.rhow[k + 1],
+                        u_top(p, F, i, j, k), p.rhow[k], u_top(p, F, i, j, k - 1), p.one_d_rhou[k]);
+        ut = fma_(mul_(p.dt, p.f[j]), ov_u, ut);
+        F.P[FU][c] = fma_(step, ut, LD(F.M[FU], c));
         T ov_v = T(0.25) * (LD(U, c) + LD(U, c + sx) + LD(U, c - sy) + LD(U, c + sx - sy));
-        T vt = -p.dtx * (v_east(p, F, i, j, k) - v_east(p, F, i - 1, j, k)) -
-               p.dty * (v_north(p, F, i, j, k) - v_north(p, F, i, j - 1, k)) -
-               DTZ * (p.rhow[k + 1] * v_top(p, F, i, j, k) - p.rhow[k] * v_top(p, F, i, j, k - 1)) *
-                   p.one_d_rhou[k] -
-               p.dt * p.f[j] * ov_v;
-        F.P[FV][c] = LD(F.M[FV], c) + step * vt;
+        T vt = flux_div(p.dtx, v_east(p, F, i, j, k) - v_east(p, F, i - 1, j, k), p.dty,
+                        v_north(p, F, i, j, k) - v_north(p, F, i, j - 1, k), DTZ, p.rhow[k + 1],
+                        v_top(p, F, i, j, k), p.rhow[k], v_top(p, F, i, j, k - 1), p.one_d_rhou[k]);
+        vt = fma_(-mul_(p.dt, p.f[j]), ov_v, vt);
+        F.P[FV][c] = fma_(step, vt, LD(F.M[FV], c));
     }
     if ((what & ADV_WB) && k >= 2) {  // buoyancy overwrite, advection.cpp:329-337
         const T *TH = F.cur[FTH];
@@ -445,35 +496,35 @@ __global__ void __launch_bounds__(128) k_advect(KParams<T> p, KFields<T> F, T st
             b1 = LD(TH, c - 1) / p.tbv[k - 1];
         } else {
             const T *QV = F.cur[FQV], *QC = F.cur[FQC], *QR = F.cur[FQR];
-            b0 = LD(TH, c) / p.tbv[k] + T(0.61) * LD(QV, c) - LD(QC, c) - LD(QR, c);
-            b1 = LD(TH, c - 1) / p.tbv[k - 1] + T(0.61) * LD(QV, c - 1) - LD(QC, c - 1) - LD(QR, c - 1);
+            b0 = buoy_moist(LD(TH, c), p.tbv[k], LD(QV, c), LD(QC, c), LD(QR, c));
+            b1 = buoy_moist(LD(TH, c - 1), p.tbv[k - 1], LD(QV, c - 1), LD(QC, c - 1), LD(QR, c - 1));
             if (p.ice) {  // buoyancy_cold_micro (advection.cpp:56-58)
                 const T *QI = F.cur[FQI], *QS = F.cur[FQS];
                 b0 = b0 - LD(QI, c) - LD(QS, c);
                 b1 = b1 - LD(QI, c - 1) - LD(QS, c - 1);
             }
         }
-        F.P[FW][c] = LD(F.M[FW], c) + sdtg * (b0 + b1);
+        F.P[FW][c] = fma_(sdtg, add_(b0, b1), LD(F.M[FW], c));
     }
     if (what & ADV_TH)  // advection.cpp:366-370
-        F.P[FTH][c] = LD(F.M[FTH], c) + step * s_tend(p, F, F.cur[FTH], F.bar[3], p.tb, i, j, k);
+        F.P[FTH][c] = fma_(step, s_tend(p, F, F.cur[FTH], F.bar[3], p.tb, i, j, k), LD(F.M[FTH], c));
     if ((what & ADV_Q) && (what & ADV_QVONLY)) {  // advect_qv, advection.cpp:577-601
-        F.P[FQV][c] = LD(F.M[FQV], c) + step * s_tend(p, F, F.cur[FQV], F.bar[4], p.qb, i, j, k);
+        F.P[FQV][c] = fma_(step, s_tend(p, F, F.cur[FQV], F.bar[4], p.qb, i, j, k), LD(F.M[FQV], c));
     } else if (what & ADV_Q) {  // advection.cpp:466-497
         if (p.rf == 1 && !p.ice) {
             const T *QR = F.cur[FQR];
             F.vt[c] = fall_speed_point(p, LD(QR, c), k);
             if (k == 1) F.vt[c - 1] = fall_speed_point(p, LD(QR, c), 1);
         }
-        T qv = LD(F.M[FQV], c) + step * s_tend(p, F, F.cur[FQV], F.bar[4], p.qb, i, j, k);
-        T qc = LD(F.M[FQC], c) + step * s_tend(p, F, F.cur[FQC], (const T *)nullptr, (const T *)nullptr, i, j, k);
-        T tr = -p.dtx * (s_east(p, F, F.cur[FQR], (const T *)nullptr, i, j, k) -
-                         s_east(p, F, F.cur[FQR], (const T *)nullptr, i - 1, j, k)) -
-               p.dty * (s_north(p, F, F.cur[FQR], (const T *)nullptr, i, j, k) -
-                        s_north(p, F, F.cur[FQR], (const T *)nullptr, i, j - 1, k)) -
-               DTZ * (p.rhow[k + 1] * r_top(p, F, i, j, k) - p.rhow[k] * r_top(p, F, i, j, k - 1)) *
-                   p.one_d_rhou[k];
-        T qr = LD(F.M[FQR], c) + step * tr;
+        T qv = fma_(step, s_tend(p, F, F.cur[FQV], F.bar[4], p.qb, i, j, k), LD(F.M[FQV], c));
+        T qc = fma_(step, s_tend(p, F, F.cur[FQC], (const T *)nullptr, (const T *)nullptr, i, j, k), LD(F.M[FQC], c));
+        T tr = flux_div(p.dtx, s_east(p, F, F.cur[FQR], (const T *)nullptr, i, j, k) -
+                                   s_east(p, F, F.cur[FQR], (const T *)nullptr, i - 1, j, k),
+                        p.dty, s_north(p, F, F.cur[FQR], (const T *)nullptr, i, j, k) -
+                                   s_north(p, F, F.cur[FQR], (const T *)nullptr, i, j - 1, k),
+                        DTZ, p.rhow[k + 1], r_top(p, F, i, j, k), p.rhow[k], r_top(p, F, i, j, k - 1),
+                        p.one_d_rhou[k]);
+        T qr = fma_(step, tr, LD(F.M[FQR], c));
         if (what & ADV_ZERO) {  // zero_moisture on this point (microphysics.cpp:675-700)
             unsigned char bits = 0;
             if (qc < 0) { qc = 0; bits |= 2; }
@@ -512,8 +563,8 @@ __global__ void k_base_tables(KParams<T> p, const T *ub, const T *vb, const T *w
         tab[(BT_C6_UB + r) * nz + k] = face5<T>(a, a, a, a, a, a, T(1));
         if (k >= 1 && k <= nz - 3) {
             const T am1 = hsrc[r][k - 1], a0 = a, a1 = hsrc[r][k + 1], a2 = hsrc[r][k + 2];
-            tab[(BT_C4_UB + 2 * r) * nz + k] = W<T>::c7_12 * (a1 + a0) - W<T>::c1_12 * (a2 + am1);
-            tab[(BT_U3_UB + 2 * r) * nz + k] = (a2 - am1) - T(3.0) * (a1 - a0);
+            tab[(BT_C4_UB + 2 * r) * nz + k] = fma_(-W<T>::c1_12, add_(a2, am1), mul_(W<T>::c7_12, add_(a1, a0)));
+            tab[(BT_U3_UB + 2 * r) * nz + k] = fma_(T(-3.0), sub_(a1, a0), sub_(a2, am1));
         } else {
             tab[(BT_C4_UB + 2 * r) * nz + k] = T(0);
             tab[(BT_U3_UB + 2 * r) * nz + k] = T(0);
@@ -530,7 +581,7 @@ __global__ void k_base_tables(KParams<T> p, const T *ub, const T *vb, const T *w
 template <typename T>
 __device__ __forceinline__ T face3_tab(const KParams<T> &p, int rc4, int k, T sign)
 {
-    return BTAB(rc4, k) + W<T>::c1_12 * sign * BTAB(rc4 + 1, k);
+    return fma_(mul_(W<T>::c1_12, sign), BTAB(rc4 + 1, k), BTAB(rc4, k));
 }
 
 template <typename T>
@@ -541,7 +592,7 @@ __device__ T u_east_ub(const KParams<T> &p, const KFields<T> &F, int i, int j, i
     T ua = T(0.5) * (LD(U, c + s) + LD(U, c));
     T uba = BTAB(BT_UA, k);
     T ue = f5i(U, p, i, j, k, sgn(uba + ua));
-    return ua * BTAB(BT_C6_UB, k) + (uba + ua) * ue;
+    return flux2(ua, BTAB(BT_C6_UB, k), (uba + ua), ue);
 }
 template <typename T>
 __device__ T u_north_ub(const KParams<T> &p, const KFields<T> &F, int i, int j, int k)
@@ -551,7 +602,7 @@ __device__ T u_north_ub(const KParams<T> &p, const KFields<T> &F, int i, int j, 
     T va = T(0.5) * (LD(V, a) + LD(V, b));
     T vba = BTAB(BT_VA, k);
     T un = f5j(U, p, i, j, k, sgn(vba + va));
-    return va * BTAB(BT_C6_UB, k) + (vba + va) * un;
+    return flux2(va, BTAB(BT_C6_UB, k), (vba + va), un);
 }
 template <typename T>
 __device__ T u_top_ub(const KParams<T> &p, const KFields<T> &F, int i, int j, int k)
@@ -569,7 +620,7 @@ __device__ T u_top_ub(const KParams<T> &p, const KFields<T> &F, int i, int j, in
         ut = f3k(U, p, i, j, k, sgn(wba + wa));
         ubt = face3_tab(p, BT_C4_UB, k, sgn(wa));
     }
-    return wa * ubt + (wba + wa) * ut;
+    return flux2(wa, ubt, wba + wa, ut);
 }
 template <typename T>
 __device__ T v_east_ub(const KParams<T> &p, const KFields<T> &F, int i, int j, int k)
@@ -579,7 +630,7 @@ __device__ T v_east_ub(const KParams<T> &p, const KFields<T> &F, int i, int j, i
     T ua = T(0.5) * (LD(U, a) + LD(U, b));
     T uba = BTAB(BT_UA, k);
     T ve = f5i(V, p, i, j, k, sgn(uba + ua));
-    return ua * BTAB(BT_C6_VB, k) + (uba + ua) * ve;
+    return flux2(ua, BTAB(BT_C6_VB, k), (uba + ua), ve);
 }
 template <typename T>
 __device__ T v_north_ub(const KParams<T> &p, const KFields<T> &F, int i, int j, int k)
@@ -589,7 +640,7 @@ __device__ T v_north_ub(const KParams<T> &p, const KFields<T> &F, int i, int j, 
     T va = T(0.5) * (LD(V, c + p.nz) + LD(V, c));
     T vba = BTAB(BT_VA, k);
     T vn = f5j(V, p, i, j, k, sgn(vba + va));
-    return va * BTAB(BT_C6_VB, k) + (vba + va) * vn;
+    return flux2(va, BTAB(BT_C6_VB, k), (vba + va), vn);
 }
 template <typename T>
 __device__ T v_top_ub(const KParams<T> &p, const KFields<T> &F, int i, int j, int k)
@@ -607,7 +658,7 @@ __device__ T v_top_ub(const KParams<T> &p, const KFields<T> &F, int i, int j, in
         vt = f3k(V, p, i, j, k, sgn(wba + wa));
         vbt = face3_tab(p, BT_C4_VB, k, sgn(wa));
     }
-    return wa * vbt + (wba + wa) * vt;
+    return flux2(wa, vbt, wba + wa, vt);
 }
 // scalar faces; brow = basic-state row offset (0: theta, 1: qv) or -1 (none)
 template <typename T>
@@ -618,7 +669,7 @@ __device__ T s_east_ub(const KParams<T> &p, const KFields<T> &F, const T *s, int
     T ut = BTAB(BT_UB, k) + u1;
     T se = f5i(s, p, i, j, k, sgn(ut));
     if (brow < 0) return ut * se;
-    return u1 * BTAB(BT_C6_THB + brow, k) + ut * se;
+    return flux2(u1, BTAB(BT_C6_THB + brow, k), ut, se);
 }
 template <typename T>
 __device__ T s_north_ub(const KParams<T> &p, const KFields<T> &F, const T *s, int brow, int i, int j, int k)
@@ -628,7 +679,7 @@ __device__ T s_north_ub(const KParams<T> &p, const KFields<T> &F, const T *s, in
     T vt = BTAB(BT_VB, k) + v1;
     T sn = f5j(s, p, i, j, k, sgn(vt));
     if (brow < 0) return vt * sn;
-    return v1 * BTAB(BT_C6_THB + brow, k) + vt * sn;
+    return flux2(v1, BTAB(BT_C6_THB + brow, k), vt, sn);
 }
 template <typename T>
 __device__ T s_top_ub(const KParams<T> &p, const KFields<T> &F, const T *s, int brow, int i, int j, int k)
@@ -646,7 +697,7 @@ __device__ T s_top_ub(const KParams<T> &p, const KFields<T> &F, const T *s, int 
         if (brow >= 0) bt = face3_tab(p, BT_C4_THB + 2 * brow, k, sgn(w1));
     }
     if (brow < 0) return wt * st;
-    return w1 * bt + wt * st;
+    return flux2(w1, bt, wt, st);
 }
 template <typename T>
 __device__ T r_top_ub(const KParams<T> &p, const KFields<T> &F, int i, int j, int k)
@@ -811,19 +862,19 @@ __device__ void advect_tile_body(const KParams<T> &p, const KFields<T> &F, int b
         const int oe = ((a + 1) * TJ + b) * nz + k, ow = (a * TJ + b) * nz + k;
         const int on = (a * (TJ + 1) + b + 1) * nz + k, os = (a * (TJ + 1) + b) * nz + k;
         const int ot = (a * TJ + b) * nz + k;
+        auto tend = [&](int f) {
+            return flux_div(p.dtx, E[f * sE + oe] - E[f * sE + ow], p.dty, Nf[f * sN + on] - Nf[f * sN + os], DTZ,
+                            p.rhow[k + 1], Tf[f * sT + ot], p.rhow[k], Tf[f * sT + ot - 1], p.one_d_rhou[k]);
+        };
         if (what & ADV_UV) {
             const T *U = F.cur[FU], *V = F.cur[FV];
             const int sy = nz, sx = p.ny * nz;
             T ov_u = T(0.25) * (LD(V, cix) + LD(V, cix + sy) + LD(V, cix - sx) + LD(V, cix - sx + sy));
-            T ut = -p.dtx * (E[oe] - E[ow]) - p.dty * (Nf[on] - Nf[os]) -
-                   DTZ * (p.rhow[k + 1] * Tf[ot] - p.rhow[k] * Tf[ot - 1]) * p.one_d_rhou[k] +
-                   p.dt * p.f[j] * ov_u;
-            F.P[FU][cix] = LD(F.M[FU], cix) + step * ut;
+            const T ut = fma_(mul_(p.dt, p.f[j]), ov_u, tend(0));
+            F.P[FU][cix] = fma_(step, ut, LD(F.M[FU], cix));
             T ov_v = T(0.25) * (LD(U, cix) + LD(U, cix + sx) + LD(U, cix - sy) + LD(U, cix + sx - sy));
-            T vt = -p.dtx * (E[sE + oe] - E[sE + ow]) - p.dty * (Nf[sN + on] - Nf[sN + os]) -
-                   DTZ * (p.rhow[k + 1] * Tf[sT + ot] - p.rhow[k] * Tf[sT + ot - 1]) * p.one_d_rhou[k] -
-                   p.dt * p.f[j] * ov_v;
-            F.P[FV][cix] = LD(F.M[FV], cix) + step * vt;
+            const T vt = fma_(-mul_(p.dt, p.f[j]), ov_v, tend(1));
+            F.P[FV][cix] = fma_(step, vt, LD(F.M[FV], cix));
         }
         if ((what & ADV_WB) && k >= 2) {
             const T *TH = F.cur[FTH];
@@ -833,29 +884,21 @@ __device__ void advect_tile_body(const KParams<T> &p, const KFields<T> &F, int b
                 b1 = LD(TH, cix - 1) / p.tbv[k - 1];
             } else {
                 const T *QV = F.cur[FQV], *QC = F.cur[FQC], *QR = F.cur[FQR];
-                b0 = LD(TH, cix) / p.tbv[k] + T(0.61) * LD(QV, cix) - LD(QC, cix) - LD(QR, cix);
-                b1 = LD(TH, cix - 1) / p.tbv[k - 1] + T(0.61) * LD(QV, cix - 1) - LD(QC, cix - 1) - LD(QR, cix - 1);
+                b0 = buoy_moist(LD(TH, cix), p.tbv[k], LD(QV, cix), LD(QC, cix), LD(QR, cix));
+                b1 = buoy_moist(LD(TH, cix - 1), p.tbv[k - 1], LD(QV, cix - 1), LD(QC, cix - 1), LD(QR, cix - 1));
                 if (p.ice) {  // buoyancy_cold_micro (advection.cpp:56-58)
                     const T *QI = F.cur[FQI], *QS = F.cur[FQS];
                     b0 = b0 - LD(QI, cix) - LD(QS, cix);
                     b1 = b1 - LD(QI, cix - 1) - LD(QS, cix - 1);
                 }
             }
-            F.P[FW][cix] = LD(F.M[FW], cix) + sdtg * (b0 + b1);
+            F.P[FW][cix] = fma_(sdtg, add_(b0, b1), LD(F.M[FW], cix));
         }
-        auto tend = [&](int f) {
-            return -p.dtx * (E[f * sE + oe] - E[f * sE + ow]) - p.dty * (Nf[f * sN + on] - Nf[f * sN + os]) -
-                   DTZ * (p.rhow[k + 1] * Tf[f * sT + ot] - p.rhow[k] * Tf[f * sT + ot - 1]) * p.one_d_rhou[k];
-        };
         const T *Wc = F.cur[FW];
         if (what & ADV_TH) {
-            T t = tend(2);
-            T zab = T(0.50) *
-                    (p.rhow[k + 1] * LD(Wc, cix + 1) * (p.tb[k + 1] - p.tb[k]) +
-                     p.rhow[k] * LD(Wc, cix) * (p.tb[k] - p.tb[k - 1])) *
-                    p.one_d_rhou[k];
-            t = t - DTZ * zab;
-            F.P[FTH][cix] = LD(F.M[FTH], cix) + step * t;
+            const T t = sub_base(tend(2), DTZ, p.rhow[k + 1], LD(Wc, cix + 1), p.tb[k + 1] - p.tb[k], p.rhow[k],
+                                 LD(Wc, cix), p.tb[k] - p.tb[k - 1], p.one_d_rhou[k]);
+            F.P[FTH][cix] = fma_(step, t, LD(F.M[FTH], cix));
         }
         if (what & ADV_Q) {
             if (p.rf == 1 && !p.ice && !(what & ADV_QVONLY)) {
@@ -863,15 +906,11 @@ __device__ void advect_tile_body(const KParams<T> &p, const KFields<T> &F, int b
                 F.vt[cix] = fall_speed_point(p, LD(QR, cix), k);
                 if (k == 1) F.vt[cix - 1] = fall_speed_point(p, LD(QR, cix), 1);
             }
-            T tv = tend(3);
-            T zab = T(0.50) *
-                    (p.rhow[k + 1] * LD(Wc, cix + 1) * (p.qb[k + 1] - p.qb[k]) +
-                     p.rhow[k] * LD(Wc, cix) * (p.qb[k] - p.qb[k - 1])) *
-                    p.one_d_rhou[k];
-            tv = tv - DTZ * zab;
-            T qv = LD(F.M[FQV], cix) + step * tv;
-            T qc = LD(F.M[FQC], cix) + step * tend(4);
-            T qr = LD(F.M[FQR], cix) + step * tend(5);
+            const T tv = sub_base(tend(3), DTZ, p.rhow[k + 1], LD(Wc, cix + 1), p.qb[k + 1] - p.qb[k], p.rhow[k],
+                                  LD(Wc, cix), p.qb[k] - p.qb[k - 1], p.one_d_rhou[k]);
+            T qv = fma_(step, tv, LD(F.M[FQV], cix));
+            T qc = fma_(step, tend(4), LD(F.M[FQC], cix));
+            T qr = fma_(step, tend(5), LD(F.M[FQR], cix));
             if (what & ADV_ZERO) {
                 unsigned char bits = 0;
                 if (qc < 0) { qc = 0; bits |= 2; }

@@ -172,7 +172,7 @@ __device__ __forceinline__ Q4 aq_east(const KParams<float> &p, const S &src, con
             const float ua = 0.5f * (up.v[e] + u0.v[e]);
             const float ue = face5<float>(x[0].v[e], x[1].v[e], x[2].v[e], x[3].v[e], x[4].v[e], x[5].v[e],
                                           sgn(uba.v[e] + ua));
-            r.v[e] = ua * c6.v[e] + (uba.v[e] + ua) * ue;
+            r.v[e] = flux2(ua, c6.v[e], (uba.v[e] + ua), ue);
         }
     } else if (FK == 1) {
         const Q4 ua_ = src.ld4(FU, c, 1, 0), ub_ = src.ld4(FU, c, 1, -1), uba = lds4(tab + BT_UA * nz + k0),
@@ -182,7 +182,7 @@ __device__ __forceinline__ Q4 aq_east(const KParams<float> &p, const S &src, con
             const float ua = 0.5f * (ua_.v[e] + ub_.v[e]);
             const float ve = face5<float>(x[0].v[e], x[1].v[e], x[2].v[e], x[3].v[e], x[4].v[e], x[5].v[e],
                                           sgn(uba.v[e] + ua));
-            r.v[e] = ua * c6.v[e] + (uba.v[e] + ua) * ve;
+            r.v[e] = flux2(ua, c6.v[e], (uba.v[e] + ua), ve);
         }
     } else {
         constexpr int BR = aq_brow(FK);
@@ -194,7 +194,7 @@ __device__ __forceinline__ Q4 aq_east(const KParams<float> &p, const S &src, con
             const float se = face5<float>(x[0].v[e], x[1].v[e], x[2].v[e], x[3].v[e], x[4].v[e], x[5].v[e],
                                           sgn(ut));
             if (BR < 0) r.v[e] = ut * se;
-            else r.v[e] = u1.v[e] * c6.v[e] + ut * se;
+            else r.v[e] = flux2(u1.v[e], c6.v[e], ut, se);
         }
     }
     return r;
@@ -219,7 +219,7 @@ __device__ __forceinline__ Q4 aq_north(const KParams<float> &p, const S &src, co
             const float va = 0.5f * (va_.v[e] + vb_.v[e]);
             const float un = face5<float>(x[0].v[e], x[1].v[e], x[2].v[e], x[3].v[e], x[4].v[e], x[5].v[e],
                                           sgn(vba.v[e] + va));
-            r.v[e] = va * c6.v[e] + (vba.v[e] + va) * un;
+            r.v[e] = flux2(va, c6.v[e], (vba.v[e] + va), un);
         }
     } else if (FK == 1) {
         const Q4 vp = src.ld4(FV, c, 0, 1), v0 = src.ld4(FV, c, 0, 0), vba = lds4(tab + BT_VA * nz + k0),
@@ -229,7 +229,7 @@ __device__ __forceinline__ Q4 aq_north(const KParams<float> &p, const S &src, co
             const float va = 0.5f * (vp.v[e] + v0.v[e]);
             const float vn = face5<float>(x[0].v[e], x[1].v[e], x[2].v[e], x[3].v[e], x[4].v[e], x[5].v[e],
                                           sgn(vba.v[e] + va));
-            r.v[e] = va * c6.v[e] + (vba.v[e] + va) * vn;
+            r.v[e] = flux2(va, c6.v[e], (vba.v[e] + va), vn);
         }
     } else {
         constexpr int BR = aq_brow(FK);
@@ -241,7 +241,7 @@ __device__ __forceinline__ Q4 aq_north(const KParams<float> &p, const S &src, co
             const float sn = face5<float>(x[0].v[e], x[1].v[e], x[2].v[e], x[3].v[e], x[4].v[e], x[5].v[e],
                                           sgn(vt));
             if (BR < 0) r.v[e] = vt * sn;
-            else r.v[e] = v1.v[e] * c6.v[e] + vt * sn;
+            else r.v[e] = flux2(v1.v[e], c6.v[e], vt, sn);
         }
     }
     return r;
@@ -286,7 +286,7 @@ __device__ __forceinline__ void aq_east_row(const KParams<float> &p, const KFiel
                 const float ua = 0.5f * (up.v[e] + u0.v[e]);
                 const float ue = face5<float>(x[0].v[e], x[1].v[e], x[2].v[e], x[3].v[e], x[4].v[e], x[5].v[e],
                                               sgn(ubar.v[e] + ua));
-                r.v[e] = ua * c6.v[e] + (ubar.v[e] + ua) * ue;
+                r.v[e] = flux2(ua, c6.v[e], (ubar.v[e] + ua), ue);
             }
             u0 = up;
         } else if (FK == 1) {
@@ -296,7 +296,7 @@ __device__ __forceinline__ void aq_east_row(const KParams<float> &p, const KFiel
                 const float ua = 0.5f * (ua_.v[e] + ub_.v[e]);
                 const float ve = face5<float>(x[0].v[e], x[1].v[e], x[2].v[e], x[3].v[e], x[4].v[e], x[5].v[e],
                                               sgn(ubar.v[e] + ua));
-                r.v[e] = ua * c6.v[e] + (ubar.v[e] + ua) * ve;
+                r.v[e] = flux2(ua, c6.v[e], (ubar.v[e] + ua), ve);
             }
         } else {
             const Q4 u1 = ldg4(U, ca + sx);
@@ -306,7 +306,7 @@ __device__ __forceinline__ void aq_east_row(const KParams<float> &p, const KFiel
                 const float se = face5<float>(x[0].v[e], x[1].v[e], x[2].v[e], x[3].v[e], x[4].v[e], x[5].v[e],
                                               sgn(ut));
                 if (BR < 0) r.v[e] = ut * se;
-                else r.v[e] = u1.v[e] * c6.v[e] + ut * se;
+                else r.v[e] = flux2(u1.v[e], c6.v[e], ut, se);
             }
         }
         sts4(E + a * TJ * nz, r);
@@ -350,7 +350,7 @@ __device__ __forceinline__ void aq_north_row(const KParams<float> &p, const KFie
                 const float va = 0.5f * (va_.v[e] + vb_.v[e]);
                 const float un = face5<float>(x[0].v[e], x[1].v[e], x[2].v[e], x[3].v[e], x[4].v[e], x[5].v[e],
                                               sgn(vbar.v[e] + va));
-                r.v[e] = va * c6.v[e] + (vbar.v[e] + va) * un;
+                r.v[e] = flux2(va, c6.v[e], (vbar.v[e] + va), un);
             }
         } else if (FK == 1) {
             const Q4 vp = ldg4(V, cb + sy);
@@ -359,7 +359,7 @@ __device__ __forceinline__ void aq_north_row(const KParams<float> &p, const KFie
                 const float va = 0.5f * (vp.v[e] + v0.v[e]);
                 const float vn = face5<float>(x[0].v[e], x[1].v[e], x[2].v[e], x[3].v[e], x[4].v[e], x[5].v[e],
                                               sgn(vbar.v[e] + va));
-                r.v[e] = va * c6.v[e] + (vbar.v[e] + va) * vn;
+                r.v[e] = flux2(va, c6.v[e], (vbar.v[e] + va), vn);
             }
             v0 = vp;
         } else {
@@ -370,7 +370,7 @@ __device__ __forceinline__ void aq_north_row(const KParams<float> &p, const KFie
                 const float sn = face5<float>(x[0].v[e], x[1].v[e], x[2].v[e], x[3].v[e], x[4].v[e], x[5].v[e],
                                               sgn(vt));
                 if (BR < 0) r.v[e] = vt * sn;
-                else r.v[e] = v1.v[e] * c6.v[e] + vt * sn;
+                else r.v[e] = flux2(v1.v[e], c6.v[e], vt, sn);
             }
         }
         sts4(N + b * nz, r);
@@ -406,9 +406,9 @@ __device__ __forceinline__ Q4 aq_top(const KParams<float> &p, const S &src, cons
                     xbt = tab[H2 * nz + k];
                 } else {
                     xt = face3<float>(x.at(e - 1), x.at(e), x.at(e + 1), x.at(e + 2), sgn(wba + wa));
-                    xbt = tab[C4 * nz + k] + W<float>::c1_12 * sgn(wa) * tab[(C4 + 1) * nz + k];
+                    xbt = fma_(mul_(W<float>::c1_12, sgn(wa)), tab[(C4 + 1) * nz + k], tab[C4 * nz + k]);
                 }
-                f = wa * xbt + (wba + wa) * xt;
+                f = flux2(wa, xbt, wba + wa, xt);
             }
             r.v[e] = f;
         }
@@ -428,11 +428,11 @@ __device__ __forceinline__ Q4 aq_top(const KParams<float> &p, const S &src, cons
                 } else {
                     st = face3<float>(x.at(e - 1), x.at(e), x.at(e + 1), x.at(e + 2), sgn(wt));
                     if (BR >= 0)
-                        bt = tab[(BT_C4_THB + 2 * BR) * nz + k] +
-                             W<float>::c1_12 * sgn(w1) * tab[(BT_C4_THB + 2 * BR + 1) * nz + k];
+                        bt = fma_(mul_(W<float>::c1_12, sgn(w1)), tab[(BT_C4_THB + 2 * BR + 1) * nz + k],
+                                  tab[(BT_C4_THB + 2 * BR) * nz + k]);
                 }
                 if (BR < 0) f = wt * st;
-                else f = w1 * bt + wt * st;
+                else f = flux2(w1, bt, wt, st);
             }
             r.v[e] = f;
         }
@@ -557,8 +557,8 @@ __device__ __forceinline__ Q4 aq_div(const KParams<float> &p, const float *sl, c
         const float tlo = e == 0 ? tb0 : tt.v[e - 1];
         const float DTZ = p.dtz * s_mu[k];
         const int kp1 = min(k + 1, nz - 1);  // level NZ-1 is padding
-        r.v[e] = -p.dtx * (ee.v[e] - ew.v[e]) - p.dty * (nn.v[e] - ns.v[e]) -
-                 DTZ * (s_rhow[kp1] * tt.v[e] - s_rhow[k] * tlo) * s_odr[k];
+        r.v[e] = flux_div(p.dtx, ee.v[e] - ew.v[e], p.dty, nn.v[e] - ns.v[e], DTZ, s_rhow[kp1], tt.v[e], s_rhow[k],
+                          tlo, s_odr[k]);
     }
     return r;
 }
@@ -636,11 +636,11 @@ __device__ __forceinline__ void advect_quad_cells(const KParams<float> &p, const
 #pragma unroll
                 for (int e = 0; e < 4; e++) {
                     const float ov_u = 0.25f * (v0.v[e] + v1.v[e] + v2.v[e] + v3.v[e]);
-                    const float ut = du.v[e] + p.dt * fj * ov_u;
-                    ru.v[e] = mu.v[e] + step * ut;
+                    const float ut = fma_(mul_(p.dt, fj), ov_u, du.v[e]);
+                    ru.v[e] = fma_(step, ut, mu.v[e]);
                     const float ov_v = 0.25f * (u0.v[e] + u1.v[e] + u2.v[e] + u3.v[e]);
-                    const float vt = dv.v[e] - p.dt * fj * ov_v;
-                    rv.v[e] = mv.v[e] + step * vt;
+                    const float vt = fma_(-mul_(p.dt, fj), ov_v, dv.v[e]);
+                    rv.v[e] = fma_(step, vt, mv.v[e]);
                 }
             }
             Q4 rw;
@@ -659,7 +659,7 @@ __device__ __forceinline__ void advect_quad_cells(const KParams<float> &p, const
                     const int k = k0 + e - 1;
                     const int kc = max(k, 0);
                     if (!p.moist) bb[e] = th.at(e - 1) / s_tbv[kc];
-                    else bb[e] = th.at(e - 1) / s_tbv[kc] + 0.61f * qv.at(e - 1) - qc.at(e - 1) - qr.at(e - 1);
+                    else bb[e] = buoy_moist(th.at(e - 1), s_tbv[kc], qv.at(e - 1), qc.at(e - 1), qr.at(e - 1));
                 }
                 if (p.ice) {  // buoyancy_cold_micro (advection.cpp:56-58): less ice, then snow
                     const Win qi = src.win(FQI, cs, 0, 0, k0);
@@ -671,7 +671,7 @@ __device__ __forceinline__ void advect_quad_cells(const KParams<float> &p, const
                 }
                 const Q4 m = ldg4(F.M[FW], c);
 #pragma unroll
-                for (int e = 0; e < 4; e++) rw.v[e] = m.v[e] + sdtg * (bb[e + 1] + bb[e]);
+                for (int e = 0; e < 4; e++) rw.v[e] = fma_(sdtg, add_(bb[e + 1], bb[e]), m.v[e]);
             }
             if (what & ADV_UV) {
                 aq_store(F.P[FU], c, k0, nz, 1, ru);
@@ -711,12 +711,9 @@ __device__ __forceinline__ void advect_quad_cells(const KParams<float> &p, const
                     const int k = k0 + e;
                     const int kl = max(k - 1, 0), kh = min(k + 1, nz - 1);
                     const float DTZ = p.dtz * s_mu[k];
-                    const float zab = 0.50f *
-                                      (s_rhow[kh] * wc.at(e + 1) * (base[kh] - base[k]) +
-                                       s_rhow[k] * wc.at(e) * (base[k] - base[kl])) *
-                                      s_odr[k];
-                    const float t = d.v[e] - DTZ * zab;
-                    float v = m.v[e] + step * t;
+                    const float t = sub_base(d.v[e], DTZ, s_rhow[kh], wc.at(e + 1), base[kh] - base[k], s_rhow[k],
+                                             wc.at(e), base[k] - base[kl], s_odr[k]);
+                    float v = fma_(step, t, m.v[e]);
                     if (fi == 1 && (what & ADV_ZERO)) {
                         const float qbar = tab[BT_QB * nz + k];
                         if (v + qbar + s_qb[k] < 0) {
@@ -759,8 +756,8 @@ __device__ __forceinline__ void advect_quad_cells(const KParams<float> &p, const
             unsigned char bits[4] = {0, 0, 0, 0};
 #pragma unroll
             for (int e = 0; e < 4; e++) {
-                float qc = mc.v[e] + step * dc.v[e];
-                float qr = mr.v[e] + step * dr.v[e];
+                float qc = fma_(step, dc.v[e], mc.v[e]);
+                float qr = fma_(step, dr.v[e], mr.v[e]);
                 if (what & ADV_ZERO) {
                     if (qc < 0) { qc = 0; bits[e] |= 2; }
                     if (qr < 0) { qr = 0; bits[e] |= 4; }
@@ -809,8 +806,8 @@ __device__ __forceinline__ void advect_quad_cells(const KParams<float> &p, const
             Q4 rs, ri;
 #pragma unroll
             for (int e = 0; e < 4; e++) {
-                float qs = ms.v[e] + step * ds.v[e];
-                float qi = mi.v[e] + step * di.v[e];
+                float qs = fma_(step, ds.v[e], ms.v[e]);
+                float qi = fma_(step, di.v[e], mi.v[e]);
                 if (what & ADV_ZERO) {
                     if (qs < 0) qs = 0;
                     if (qi < 0) qi = 0;
