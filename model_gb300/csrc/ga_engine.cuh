@@ -501,6 +501,17 @@ class Engine : public EngineBase {
             kp.mean_inv = upload(inv);
         }
 
+        if (sizeof(T) == 8) {
+            const int ncol = ni * nh;
+            double *zt = dalloc<double>((size_t)ncol * (NZ - 2)), *ft = dalloc<double>((size_t)ncol * (NZ - 2));
+            if (zt && ft) {
+                k_thomas_table<<<cdiv(ncol, 128), 128>>>(ncol, NZ, kp.dx2, kp.hcoef, kp.rhou_d, kp.acoef_d, kp.ccoef_d,
+                                                         kp.vcoef_d, zt, ft);
+                kp.th_z = zt;
+                kp.th_f = ft;
+            }
+        }
+
         // ---- FFT plans and twiddles ----
         plan_i = make_fft_plan(ni);
         plan_j = make_fft_plan(nj);
@@ -535,6 +546,10 @@ class Engine : public EngineBase {
             const int ps = nl + ((1 - nl % m) % m + m) % m;
             if (2 * (size_t)ni * ps * sizeof(T2) <= (size_t)optin) psx = ps;
             else if (2 * (size_t)ni * (nl | 1) * sizeof(T2) <= (size_t)optin) psx = nl | 1;
+            // FP64: the fused kernel's nh blocks leave most of the few FP64 lanes
+            // idle (65 blocks at 128x128: 217 us a solve); the level-tiled x
+            // transforms and the table solve use every SM
+            if (sizeof(T) == 8) psx = 0;
             smem_sx = 2 * (size_t)ni * psx * sizeof(T2);
             // one radix-8 butterfly per thread: the block's passes are chains
             // of shared-memory round trips, so idle or looping threads cost time
@@ -573,7 +588,7 @@ class Engine : public EngineBase {
         if (const char *ev = std::getenv("GA_SPECTRAL_X"))  // fused x block of 1024 threads by default
             if (!std::strcmp(ev, "1024")) sx_threads = 1024;
         if (const char *ev = std::getenv("GA_POST")) post_quad = std::strcmp(ev, "column") != 0;
-        post_quad = post_quad && sizeof(T) == 4 && NZ % 4 == 0;
+        post_quad = post_quad && NZ % pq_levels<T>() == 0;
         if (const char *ev = std::getenv("GA_KESSLER")) kes_fused = std::strcmp(ev, "separate") != 0;
         if constexpr (sizeof(T) == 4) {
             smem_sxp = sx_pair_smem(kp.ni, NZ);
@@ -1230,26 +1245,25 @@ class Engine : public EngineBase {
         if (!(fl[0] | fl[1] | fl[2] | fl[3] | fl[4] | fl[5] | fl[6])) return;
         int4 a = make_int4(fl[0], fl[1], fl[2], fl[3]), b = make_int4(fl[4], fl[5], fl[6], fl[7]);
         ProfScope ps(this, PC_POST, (pcopy && kp.periodic) ? 2 : 1);
-        if constexpr (sizeof(T) == 4) {
-            if (post_quad) {
-                const long nq = NZ / 4;
-                auto go = [&](long ncols, int mode) {
+        if (post_quad) {
+            const long nq = NZ / pq_levels<T>();
+            auto go = [&](long ncols, int mode) {
+                const int nb = cdiv(ncols * nq, PQ_THREADS);
+                if constexpr (sizeof(T) == 4) {
                     if (post_kes)
-                        k_post_quad<T, true><<<cdiv(ncols * nq, PQ_THREADS), PQ_THREADS, 0, stream>>>(
-                            kp, F, a, b, (T)step, mode, d_err);
-                    else
-                        k_post_quad<T><<<cdiv(ncols * nq, PQ_THREADS), PQ_THREADS, 0, stream>>>(kp, F, a, b, (T)step,
-                                                                                            mode, d_err);
-                    launches++;
-                };
-                if (pcopy && kp.periodic) {
-                    go(6L * NY, COLS_TARGETS);
-                    go((long)(NX - 6) * NY, COLS_NONTARGETS);
-                } else {
-                    go((long)NX * NY, COLS_ALL);
+                        k_post_quad<T, true><<<nb, PQ_THREADS, 0, stream>>>(kp, F, a, b, (T)step, mode, d_err);
                 }
-                return;
+                if (!(post_kes && sizeof(T) == 4))
+                    k_post_quad<T><<<nb, PQ_THREADS, 0, stream>>>(kp, F, a, b, (T)step, mode, d_err);
+                launches++;
+            };
+            if (pcopy && kp.periodic) {
+                go(6L * NY, COLS_TARGETS);
+                go((long)(NX - 6) * NY, COLS_NONTARGETS);
+            } else {
+                go((long)NX * NY, COLS_ALL);
             }
+            return;
         }
         if (pcopy && kp.periodic) {
             k_post<T><<<cdiv(6L * NY, POST_COLS), POST_THREADS, 0, stream>>>(kp, F, 7, a, b, (T)step, COLS_TARGETS);
@@ -1666,7 +1680,8 @@ class Engine : public EngineBase {
         // FP32, Eulerian rain, non-periodic: Kessler runs inside the last
         // column pass (a periodic domain's copied columns take their own
         // rain totals, so it keeps the separate kernel)
-        const bool fuse_kes = moist && !kp.ice && kes_fused && post_quad && kp.rf == 1 && !kp.periodic;
+        const bool fuse_kes =
+            sizeof(T) == 4 && moist && !kp.ice && kes_fused && post_quad && kp.rf == 1 && !kp.periodic;
         if (moist && !fuse_kes) microphysics(false);
         int fl[9] = {};
         fl[FU] = fl[FV] = fl[FW] = fl[FTH] = PF_SPONGE | PF_VBC | PF_RAYLEIGH | PF_WRITE_M;

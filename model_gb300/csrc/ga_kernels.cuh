@@ -45,6 +45,9 @@ struct KParams {
     const double *hcoef;                        // (cos kx + cos ly) - 2 per (p,q)
     const T *acoef, *ccoef, *vcoef;             // [nz]
     const double *acoef_d, *ccoef_d, *vcoef_d, *rhou_d;  // FP64 islands
+    // FP64 contexts: the elimination of every wavenumber's system, [level][column]
+    // (columns p*nh + q, ncol = ni*nh): reciprocal pivots and upper factors, or null
+    const double *th_z, *th_f;
     double dx2;
     T rhou1;
     int low_modes;  // |p|,|q| below this solve in FP64 (FP32 contexts)
@@ -1546,6 +1549,71 @@ __device__ void thomas_column(const KParams<T> &p, typename V2<T>::t *x, A *Fw, 
     }
 }
 
+// The elimination of thomas_column for every column, once per context: its
+// reciprocal pivots z and upper factors F do not change during a run.  A solve
+// then multiplies where it divided (FP64 divisions are chains of dependent
+// operations on a pipe of two lanes an SM).
+static __global__ void k_thomas_table(int ncol, int nz, double dx2, const double *hcoef, const double *rhou,
+                                      const double *ac, const double *cc, const double *vc, double *zt, double *ft)
+{
+    const int col = blockIdx.x * blockDim.x + threadIdx.x;
+    if (col >= ncol) return;
+    const double h = hcoef[col];
+    double Fk = 0.0;
+    for (int k = 1; k < nz - 1; k++) {
+        const double bk = rhou[k] * 2.0 * h / dx2 - vc[k];
+        const double z = 1.0 / (k == 1 ? bk : bk - ac[k] * Fk);
+        Fk = cc[k] * z;
+        zt[(long)(k - 1) * ncol + col] = z;
+        ft[(long)(k - 1) * ncol + col] = Fk;
+    }
+}
+// the solve from that table; the next level's values are read before this
+// level's are written
+template <typename T2>
+__device__ __forceinline__ void thomas_column_table(T2 *x, int nz, int col, int ncol, const double *__restrict__ zt,
+                                                    const double *__restrict__ ft, double inv_size2d,
+                                                    const double *ac, bool gauge)
+{
+    double xr = 0.0, xi = 0.0, z = zt[col], a = 0.0;
+    T2 d = x[1];
+    for (int k = 1; k < nz - 1; k++) {
+        const int kn = min(k + 1, nz - 2);
+        const T2 dn = x[kn];
+        const double zn = zt[(long)(kn - 1) * ncol + col], an = ac[kn];
+        xr = (d.x * inv_size2d - a * xr) * z;
+        xi = (d.y * inv_size2d - a * xi) * z;
+        T2 o;
+        o.x = xr;
+        o.y = xi;
+        x[k] = o;
+        d = dn;
+        z = zn;
+        a = an;
+    }
+    if (gauge) {  // pressure.cpp:858-859
+        xr = xi = 0.0;
+        T2 o;
+        o.x = o.y = 0.0;
+        x[nz - 2] = o;
+    }
+    d = x[nz - 3];
+    double f = ft[(long)(nz - 4) * ncol + col];
+    for (int k = nz - 3; k >= 1; k--) {
+        const int kn = max(k - 1, 1);
+        const T2 dn = x[kn];
+        const double fn = ft[(long)(kn - 1) * ncol + col];
+        xr = d.x - f * xr;
+        xi = d.y - f * xi;
+        T2 o;
+        o.x = xr;
+        o.y = xi;
+        x[k] = o;
+        d = dn;
+        f = fn;
+    }
+}
+
 // FP32 Thomas solve of one wavenumber: the reference recurrence
 // (pressure.cpp:834-871) with the horizontal term of the diagonal hoisted and
 // one reciprocal per level instead of three divisions.
@@ -1764,8 +1832,12 @@ __device__ void thomas_body(const KParams<T> &p, typename V2<T>::t *spec, int TC
         const int col = c0 + c, pp = col / p.nh, q = col - pp * p.nh;
         T2 *x = xs + (long)c * cs - 1;
         if (sizeof(T) == 8) {
-            double Floc[PPM_MAXZ];
-            thomas_column<T, double>(p, x, Floc, col, size2d, p.rhou_d, p.acoef_d, p.ccoef_d, p.vcoef_d);
+            if (p.th_z) {
+                thomas_column_table(x, p.nz, col, ncol, p.th_z, p.th_f, 1.0 / size2d, p.acoef_d, col == 0);
+            } else {
+                double Floc[PPM_MAXZ];
+                thomas_column<T, double>(p, x, Floc, col, size2d, p.rhou_d, p.acoef_d, p.ccoef_d, p.vcoef_d);
+            }
         } else if (!low_mode(p, pp, q)) {
             const float hb = 2.0f * (float)p.hcoef[col] / (float)p.dx2;
             thomas_column_fast((float2 *)x, (float *)(fs + (long)c * cs), p.nz, hb, (float)(1.0 / size2d),
@@ -2005,23 +2077,20 @@ __device__ __forceinline__ T chain_value(const KParams<T> &p, const KFields<T> &
 // are exchanged through shared memory for the top/bottom condition.
 constexpr int POST_COLS = 8, POST_R = 4, POST_THREADS = 256;  // POST_COLS * NZ <= POST_R * POST_THREADS
 
-__device__ __forceinline__ void post_column(const int mode, const long c, const int nx, const int ny, int &i, int &j,
+__device__ __forceinline__ void post_column(const int mode, const int c, const int nx, const int ny, int &i, int &j,
                                             bool &ok)
 {
-    ok = true;
+    const int i0 = c / ny;
+    j = c - i0 * ny;
     if (mode == COLS_TARGETS) {
-        if (c >= 6L * ny) { ok = false; return; }
-        const int col = (int)(c / ny);
-        j = (int)(c % ny);
-        i = col < 3 ? col : nx - 6 + col;
+        ok = i0 < 6;
+        i = i0 < 3 ? i0 : nx - 6 + i0;
     } else if (mode == COLS_NONTARGETS) {
-        if (c >= (long)(nx - 6) * ny) { ok = false; return; }
-        i = 3 + (int)(c / ny);
-        j = (int)(c % ny);
+        ok = i0 < nx - 6;
+        i = 3 + i0;
     } else {
-        if (c >= (long)nx * ny) { ok = false; return; }
-        i = (int)(c / ny);
-        j = (int)(c % ny);
+        ok = i0 < nx;
+        i = i0;
     }
 }
 
@@ -2040,7 +2109,7 @@ __device__ void post_body(const KParams<T> &p, const KFields<T> &F, int nfields,
         const int cl = e / nz, k = e - cl * nz;
         int i = 0, j = 0;
         bool ok = false;
-        if (cl < POST_COLS) post_column(cols, c0 + cl, p.nx, p.ny, i, j, ok);
+        if (cl < POST_COLS) post_column(cols, (int)c0 + cl, p.nx, p.ny, i, j, ok);
         if (!ok) continue;
         // the chain runs at the source column (the column itself, or the
         // column a periodic target copies)
@@ -2098,7 +2167,7 @@ __device__ void post_body(const KParams<T> &p, const KFields<T> &F, int nfields,
         const int cl = e / nz, k = e - cl * nz;
         int i = 0, j = 0;
         bool ok = false;
-        if (cl < POST_COLS) post_column(cols, c0 + cl, p.nx, p.ny, i, j, ok);
+        if (cl < POST_COLS) post_column(cols, (int)c0 + cl, p.nx, p.ny, i, j, ok);
         if (!ok) continue;
         const int c = gix(p.ny, nz, i, j, k);
         const bool vbc = i >= 1 && j >= 1;

@@ -1140,6 +1140,53 @@ __device__ void thomas_T_column(T2 *x, A *Fw, int nz, A hb, A inv_s, const A *rh
     }
 }
 
+// The transposed solve from the forward elimination's table (FP64):
+// M = (L D)(I + F), so M^T z = y is g_k = y_k - F_(k-1) g_(k-1) upward, then
+// z_k = (g_k - a_(k+1) z_(k+1)) / pivot_k downward.  The mean mode's rows
+// 1..K-1 are the leading block of the same factors; z_K = 0.
+template <typename T2>
+__device__ __forceinline__ void thomas_T_column_table(T2 *x, int nz, int col, int ncol, const double *__restrict__ zt,
+                                                      const double *__restrict__ ft, double inv_s, const double *ac,
+                                                      bool gauge)
+{
+    const int K = gauge ? nz - 3 : nz - 2;
+    double gr = 0.0, gi = 0.0, f = 0.0;
+    T2 d = x[1];
+    for (int k = 1; k <= K; k++) {
+        const T2 dn = x[min(k + 1, K)];
+        const double fn = ft[(long)(k - 1) * ncol + col];
+        gr = d.x * inv_s - f * gr;
+        gi = d.y * inv_s - f * gi;
+        T2 o;
+        o.x = gr;
+        o.y = gi;
+        x[k] = o;
+        d = dn;
+        f = fn;
+    }
+    double zr = 0.0, zi = 0.0, a = 0.0, z = zt[(long)(K - 1) * ncol + col];
+    d = x[K];
+    for (int k = K; k >= 1; k--) {
+        const int kn = max(k - 1, 1);
+        const T2 dn = x[kn];
+        const double zn = zt[(long)(kn - 1) * ncol + col], an = ac[k];
+        zr = (d.x - a * zr) * z;
+        zi = (d.y - a * zi) * z;
+        T2 o;
+        o.x = zr;
+        o.y = zi;
+        x[k] = o;
+        d = dn;
+        z = zn;
+        a = an;
+    }
+    if (gauge) {
+        T2 o;
+        o.x = o.y = 0.0;
+        x[nz - 2] = o;
+    }
+}
+
 // FP32 transposed solve of one wavenumber (not the mean mode): the recurrence
 // of thomas_T_column with one reciprocal per level
 __device__ __forceinline__ void thomas_T_column_fast(float2 *x, float *Fw, int nz, float hb, float inv_s,
@@ -1303,7 +1350,9 @@ __global__ void k_thomas_adj(KParams<T> p, typename V2<T>::t *spec, int TC)
         const int col = c0 + c;
         T2 *x = xs + (long)c * cs - 1;
         if (col == 0 && mean_block) continue;
-        if (sizeof(T) == 8 || col == 0) {
+        if (sizeof(T) == 8 && p.th_z) {
+            thomas_T_column_table(x, p.nz, col, ncol, p.th_z, p.th_f, inv_s, p.acoef_d, col == 0);
+        } else if (sizeof(T) == 8 || col == 0) {
             double Floc[PPM_MAXZ];
             thomas_T_column<T2, double>(x, Floc, p.nz, 2.0 * p.hcoef[col] / p.dx2, inv_s, p.rhou_d,
                                         p.acoef_d, p.ccoef_d, p.vcoef_d, col == 0);

@@ -940,11 +940,37 @@ __global__ void __launch_bounds__(AQ_THREADS, MB)
 
 // ---------------------------------------------------------------------------
 // k_post_quad: the column post-processing of k_post, expression for
-// expression.  A column's bottom and top conditions copy level 1 to 0 and
-// NZ-2 to NZ-1, both inside one quad, so every thread reads and writes only
-// its own points and the fields go one after another without a barrier.
+// expression, on 16-byte runs of a column.  A column's bottom and top
+// conditions copy level 1 to 0 and NZ-2 to NZ-1, both inside one run, so every
+// thread reads and writes only its own points and the fields go one after
+// another without a barrier.  FP64 (two levels; bound by latency: the column
+// kernel's index divisions and its exchange through shared memory).
 // ---------------------------------------------------------------------------
 constexpr int PQ_THREADS = 256;
+// levels per thread: 16 bytes of a column (four in FP32, two in FP64)
+template <typename T> __host__ __device__ constexpr int pq_levels() { return 16 / (int)sizeof(T); }
+template <typename T>
+struct LV {
+    T v[pq_levels<T>()];
+};
+__device__ __forceinline__ LV<float> ldv(const float *a)
+{
+    const float4 t = __ldg(reinterpret_cast<const float4 *>(a));
+    return LV<float>{{t.x, t.y, t.z, t.w}};
+}
+__device__ __forceinline__ LV<double> ldv(const double *a)
+{
+    const double2 t = __ldg(reinterpret_cast<const double2 *>(a));
+    return LV<double>{{t.x, t.y}};
+}
+__device__ __forceinline__ void stv(float *a, const LV<float> &q)
+{
+    *reinterpret_cast<float4 *>(a) = make_float4(q.v[0], q.v[1], q.v[2], q.v[3]);
+}
+__device__ __forceinline__ void stv(double *a, const LV<double> &q)
+{
+    *reinterpret_cast<double2 *>(a) = make_double2(q.v[0], q.v[1]);
+}
 
 // item w: column w / (NZ/4) of the enumeration `cols`, level quad w % (NZ/4).
 // KES: the step's last pass with Kessler (run_kessler_microphysics,
@@ -958,12 +984,12 @@ template <typename T, bool KES = false>
 __device__ __forceinline__ void post_quad_body(const KParams<T> &p, const KFields<T> &F, int4 fl0, int4 fl1, T step,
                                                int cols, long w, int *err = nullptr)
 {
-    static_assert(sizeof(T) == 4, "four-level kernels are FP32");
-    const int nz = p.nz, NQ = nz >> 2, sx = p.ny * nz, sy = nz;
-    const int q = (int)(w % NQ), k0 = 4 * q;
+    constexpr int L = pq_levels<T>();
+    const int nz = p.nz, NQ = nz / L, sx = p.ny * nz, sy = nz;
+    const int col = (int)w / NQ, q = (int)w - col * NQ, k0 = L * q;  // fewer than 2^31 points
     int i = 0, j = 0;
     bool ok = false;
-    post_column(cols, w / NQ, p.nx, p.ny, i, j, ok);
+    post_column(cols, col, p.nx, p.ny, i, j, ok);
     if (!ok) return;
     const int flv[7] = {fl0.x, fl0.y, fl0.z, fl0.w, fl1.x, fl1.y, fl1.z};
     // the chain runs at the source column (the column itself, or the column a
@@ -978,33 +1004,34 @@ __device__ __forceinline__ void post_quad_body(const KParams<T> &p, const KField
     const bool hW = !p.periodic && j >= 1 && si >= p.wb && si < p.we;
     const bool hS = si >= 1 && j >= p.sb && j < p.se;
     const bool hN = si >= 1 && j >= p.nb && j < p.ne;
-    const float cE = hE ? p.ce[si - p.eb] : 0.f, cW = hW ? p.cw[si - p.wb] : 0.f;
-    const float cS = hS ? p.cs[j - p.sb] : 0.f, cN = hN ? p.cn[j - p.nb] : 0.f;
-    float dpx[4] = {0.f, 0.f, 0.f, 0.f}, dpy[4] = {0.f, 0.f, 0.f, 0.f}, dpz[4] = {0.f, 0.f, 0.f, 0.f};
+    const T cE = hE ? p.ce[si - p.eb] : T(0), cW = hW ? p.cw[si - p.wb] : T(0);
+    const T cS = hS ? p.cs[j - p.sb] : T(0), cN = hN ? p.cn[j - p.nb] : T(0);
+    T dpx[L] = {}, dpy[L] = {}, dpz[L] = {};
     if (col_in && ((flv[FU] | flv[FV] | flv[FW]) & PF_PROJECT)) {
-        const Win pc = ldwin(F.pi, cs, k0, nz);
-        const Q4 px = ldg4(F.pi, cs - sx), py = ldg4(F.pi, cs - sy);
+        const LV<T> pc = ldv(F.pi + cs), px = ldv(F.pi + cs - sx), py = ldv(F.pi + cs - sy);
+        const T pm = k0 > 0 ? LD(F.pi, cs - 1) : T(0);  // level k0-1
 #pragma unroll
-        for (int e = 0; e < 4; e++) {
-            dpx[e] = pc.at(e) - px.v[e];
-            dpy[e] = pc.at(e) - py.v[e];
-            dpz[e] = pc.at(e) - pc.at(e - 1);
+        for (int e = 0; e < L; e++) {
+            dpx[e] = pc.v[e] - px.v[e];
+            dpy[e] = pc.v[e] - py.v[e];
+            dpz[e] = pc.v[e] - (e > 0 ? pc.v[e - 1] : pm);
         }
     }
     // every field's quad is loaded before any is written (a store to one
     // field's buffer would otherwise order the next field's load after it)
-    Q4 inq[7];
+    LV<T> inq[7] = {};
 #pragma unroll
-    for (int f = 0; f < 7; ++f) inq[f] = flv[f] ? ldg4(F.P[f], cs) : Q4{{0.f, 0.f, 0.f, 0.f}};
+    for (int f = 0; f < 7; ++f)
+        if (flv[f]) inq[f] = ldv(F.P[f] + cs);
     if constexpr (KES) {
         if (col_in) {
-            const float qr0 = inq[FQR].v[0];  // level 0 before the chain (precip_rate reads it)
-            const Q4 pq = ldg4(F.pi, cs);
+            const T qr0 = inq[FQR].v[0];  // level 0 before the chain (precip_rate reads it)
+            const LV<T> pq = ldv(F.pi + cs);
 #pragma unroll
-            for (int e = 0; e < 4; e++) {
+            for (int e = 0; e < L; e++) {
                 const int k = k0 + e;
                 if (k < 1 || k >= nz - 1) continue;
-                float th = inq[FTH].v[e], qv = inq[FQV].v[e], qc = inq[FQC].v[e], qr = inq[FQR].v[e];
+                T th = inq[FTH].v[e], qv = inq[FQV].v[e], qc = inq[FQC].v[e], qr = inq[FQR].v[e];
                 if (kessler_point(th, qv, qc, qr, pq.v[e], kes_point(p, F, k, (long)cs + e),
                                   F.sat ? F.sat + cs + e : nullptr))
                     atomicExch(err, 1);
@@ -1014,30 +1041,30 @@ __device__ __forceinline__ void post_quad_body(const KParams<T> &p, const KField
                 inq[FQR].v[e] = qr;
             }
             if (q == 0 && cols != COLS_TARGETS) {
-                const double inc = (double)(p.rhow[1] * 0.5f * (F.vt[cs] + F.vt[cs + 1]) * 0.5f *
+                const double inc = (double)(p.rhow[1] * T(0.5) * (F.vt[cs] + F.vt[cs + 1]) * T(0.5) *
                                             (qr0 + inq[FQR].v[1]) * p.dt);
                 F.accrain[(long)si * p.ny + j] += inc;
             }
         }
     }
-    Q4 qb4{{0.f, 0.f, 0.f, 0.f}};
-    if ((flv[FQV] & PF_ZERO) && col_in) qb4 = ldg4(F.bar[4], cs);
+    LV<T> qb4 = {};
+    if ((flv[FQV] & PF_ZERO) && col_in) qb4 = ldv(F.bar[4] + cs);
 #pragma unroll
     for (int f = 0; f < 7; ++f) {
         const int flags = flv[f];
         if (!flags) continue;
-        const Q4 in = inq[f];
-        float ch[4];
+        const LV<T> in = inq[f];
+        T ch[L];
 #pragma unroll
-        for (int e = 0; e < 4; e++) {
+        for (int e = 0; e < L; e++) {
             const int k = k0 + e;
             const bool inner = col_in && k >= 1 && k < nz - 1;
-            float v = in.v[e];
+            T v = in.v[e];
             if (flags & PF_ZERO) {  // zero_moisture, microphysics.cpp:675-700
                 if (f == FQC || f == FQR) {
                     if (v < 0) v = 0;
                 } else if (f == FQV && inner) {
-                    const float qbar = qb4.v[e];
+                    const T qbar = qb4.v[e];
                     if (v + qbar + p.qb[k] < 0) v = -(qbar + p.qb[k]);
                 }
             }
@@ -1054,27 +1081,27 @@ __device__ __forceinline__ void post_quad_body(const KParams<T> &p, const KField
             }
             ch[e] = v;
         }
-        Q4 out;
+        LV<T> out;
 #pragma unroll
-        for (int e = 0; e < 4; e++) {
+        for (int e = 0; e < L; e++) {
             const int k = k0 + e;
-            float v = ch[e];
+            T v = ch[e];
             if ((flags & PF_VBC) && vbc) {  // boundaries.cpp:304-326
                 if (f == FW) {
-                    if (k == 0 || k == 1 || k == nz - 1) v = 0.f;
+                    if (k == 0 || k == 1 || k == nz - 1) v = T(0);
                 } else {
                     if (k == 0) v = ch[1];
-                    if (k == nz - 1) v = ch[2];
+                    if (k == nz - 1) v = ch[L - 2];
                 }
             }
             if ((flags & PF_RAYLEIGH) && f <= FTH && ray_col && k >= p.raylevel) {  // damping.cpp:1148-1177
-                const float cr = (f == FW) ? p.ray_w[k] : p.ray_u[k];
+                const T cr = (f == FW) ? p.ray_w[k] : p.ray_u[k];
                 v = v - cr * v;
             }
             out.v[e] = v;
         }
-        stg4(F.P[f] + c, out);
-        if (flags & PF_WRITE_M) stg4(F.M[f] + c, out);
+        stv(F.P[f] + c, out);
+        if (flags & PF_WRITE_M) stv(F.M[f] + c, out);
     }
 }
 
