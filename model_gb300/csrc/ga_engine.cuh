@@ -69,6 +69,8 @@ class Engine : public EngineBase {
     bool bar_uniform[6] = {false, false, false, false, false, false};
     bool btab_dirty = true;
     T *btab = nullptr, *mtab = nullptr;
+    T *bface = nullptr;  // both upwind values of the basic-state faces (FP64)
+    bool bface_tried = false;
     long long graph_launches[2] = {0, 0};
     bool use_graphs = true;
     int status = GA_OK;
@@ -559,11 +561,11 @@ class Engine : public EngineBase {
         cudaFuncSetAttribute(k_spectral_x<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
         cudaFuncSetAttribute(k_spectral_x_1k<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
         smem_adv = advect_tile_smem(adv_ti, adv_tj, NZ, sizeof(T));
-        cudaFuncSetAttribute(k_advect_tile<T, 4, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
-        cudaFuncSetAttribute(k_advect_tile<T, 2, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
-        cudaFuncSetAttribute(k_advect_tile<T, 4, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
-        cudaFuncSetAttribute(k_advect_tile<T, 4, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
-        cudaFuncSetAttribute(k_advect_tile<T, 8, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
+        cudaFuncSetAttribute(k_advect_tile<T, 4, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+        cudaFuncSetAttribute(k_advect_tile<T, 2, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+        cudaFuncSetAttribute(k_advect_tile<T, 4, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+        cudaFuncSetAttribute(k_advect_tile<T, 4, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+        cudaFuncSetAttribute(k_advect_tile<T, 8, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
         if (const char *ev = std::getenv("GA_ADVECT")) {
             if (!std::strcmp(ev, "tile")) adv_force = 1;
             else if (!std::strcmp(ev, "quad")) adv_force = 2;
@@ -626,6 +628,7 @@ class Engine : public EngineBase {
             if (g) cudaGraphExecDestroy(g);
         for (void *p : allocs) cudaFree(p);
         if (staging) cudaFree(staging);
+        if (bface) cudaFree(bface);
         if (stream2) cudaStreamSynchronize(stream2);
         if (ev_fork) cudaEventDestroy(ev_fork);
         if (ev_join) cudaEventDestroy(ev_join);
@@ -847,6 +850,23 @@ class Engine : public EngineBase {
                 launches++;
             }
         }
+        kp.bface = nullptr;
+        if constexpr (sizeof(T) == 8) {
+            if (!adv && !cfg.linear_model) {  // (without the memory for it the faces are evaluated each time)
+                const int nfb = kp.moist ? 4 : 3, src[4] = {0, 1, 3, 4};
+                if (!bface && !bface_tried && cudaMalloc(&bface, (size_t)nfb * 6 * N * sizeof(T)) != cudaSuccess) {
+                    bface = nullptr;
+                    cudaGetLastError();
+                }
+                bface_tried = true;
+                if (bface) {
+                    for (int b = 0; b < nfb; b++)
+                        k_base_faces<T><<<cdiv(N, 256), 256, 0, stream>>>(kp, bar[src[b]], b, bface);
+                    launches += nfb;
+                    kp.bface = bface;
+                }
+            }
+        }
         kp.ubase_adv = adv && !cfg.linear_model;  // the tables hold the full-velocity faces only
         kp.ubase_kes = kes;
     }
@@ -858,7 +878,8 @@ class Engine : public EngineBase {
     void launch_advect_tile(T step, T sdtg, int what)
     {
         dim3 grid(cdiv(NX - 6, TI), cdiv(NY - 6, TJ));
-        k_advect_tile<T, TI, TJ><<<grid, 256, smem_adv, stream>>>(kp, fields(), step, sdtg, what);
+        k_advect_tile<T, TI, TJ><<<grid, adv_threads<T>(), advect_tile_smem(TI, TJ, NZ, sizeof(T), what), stream>>>(
+            kp, fields(), step, sdtg, what);
     }
 
     // the four-level kernel's tiles the autotuner chooses from

@@ -241,6 +241,7 @@ class Ensemble : public EnsembleBase {
     // the step advects everything in one launch: u, v, w's buoyancy, theta
     // and the moisture
     int step_jobs() const { return moist ? 7 : 4; }
+    int step_what() const { return ADV_UV | ADV_WB | ADV_TH | (moist ? (ADV_Q | ADV_ZERO) : 0); }
     // a member's tile: chunks of up to 16 columns (many members fill the GPU)
     MarchGeom member_march(const Engine<T> &e) const { return march_geom(e.NX, e.NY, e.NZ, step_jobs(), nsm, adv_li); }
 
@@ -275,11 +276,11 @@ class Ensemble : public EnsembleBase {
         cudaMalloc(&d_err, sizeof(int));
         cudaMemset(d_err, 0, sizeof(int));
         const int optin = 200 * 1024;
-        cudaFuncSetAttribute(kb_advect<T, 4, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
-        cudaFuncSetAttribute(kb_advect<T, 2, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
-        cudaFuncSetAttribute(kb_advect<T, 4, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
-        cudaFuncSetAttribute(kb_advect<T, 4, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
-        cudaFuncSetAttribute(kb_advect<T, 8, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
+        cudaFuncSetAttribute(kb_advect<T, 4, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+        cudaFuncSetAttribute(kb_advect<T, 2, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+        cudaFuncSetAttribute(kb_advect<T, 4, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+        cudaFuncSetAttribute(kb_advect<T, 4, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+        cudaFuncSetAttribute(kb_advect<T, 8, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
         cudaFuncSetAttribute(kb_div_fft_y<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
         cudaFuncSetAttribute(kb_spectral_x<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
         cudaFuncSetAttribute(kb_ifft_y_pi<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
@@ -398,7 +399,7 @@ class Ensemble : public EnsembleBase {
                         sm = std::max(sm, march_smem(g.tj, e.NZ));
                     } else {
                         c = (long)cdiv(e.NX - 6, adv_ti) * cdiv(e.NY - 6, adv_tj);
-                        sm = std::max(sm, advect_tile_smem(adv_ti, adv_tj, e.NZ, sizeof(T)));
+                        sm = std::max(sm, advect_tile_smem(adv_ti, adv_tj, e.NZ, sizeof(T), step_what()));
                     }
                     break;
                 case EK_MIRROR: c = cdiv(2L * (e.NX + e.NY - 2) * (e.NZ - 2), 256); break;
@@ -493,7 +494,7 @@ class Ensemble : public EnsembleBase {
             cudaEventElapsedTime(&ms, ea, eb);
             return cudaGetLastError() == cudaSuccess ? ms / 3.f : 1e30f;
         };
-        const int what = ADV_UV | ADV_WB | ADV_TH | (moist ? (ADV_Q | ADV_ZERO) : 0);
+        const int what = step_what();
         const KFields<T> *F = d_f[rot];
         std::string info;
         char line[160];
@@ -674,7 +675,7 @@ class Ensemble : public EnsembleBase {
         for (int s = 0; s < 3; s++) {
             const double st = steps[s];
             KFields<T> *F = d_f[rot];
-            const int what = ADV_UV | ADV_WB | ADV_TH | (moist ? (ADV_Q | ADV_ZERO) : 0);
+            const int what = step_what();
             launch_advect(F, st, what);
             kb_mirror<T><<<grid[EK_MIRROR], 256, 0, stream>>>(d_p, F, d_pre[EK_MIRROR], nmem);
             kb_div_fft_y<T><<<grid[EK_DIVY], dim3(8, 32), smem[EK_DIVY], stream>>>(d_p, F, d_aux, d_pre[EK_DIVY],

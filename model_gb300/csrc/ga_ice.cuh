@@ -147,7 +147,7 @@ __device__ T fall_top(const KParams<T> &p, const KFields<T> &F, const T *s, cons
     T wf = wb - T(0.5) * (fall[a - 1] + fall[a]);
     T st;
     if (k == 1 || k == p.nz - 2) st = f2k(s, p, i, j, k);
-    else st = f3k(s, p, i, j, k, sgn(wf));
+    else st = f3k(s, p, i, j, k, up12(wf));
     return wf * st;
 }
 

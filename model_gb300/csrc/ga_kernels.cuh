@@ -59,6 +59,7 @@ struct KParams {
     int ubase_kes;  // THBAR, QBAR, PBAR depend on k only
     const T *btab;
     const T *mtab;  // rows of the marching advection kernel (MT_*), FP32
+    const T *bface;  // both upwind values of the basic-state faces (k_base_faces), or null
     // the linearised model (ISLINEAR): perturbation faces advected by the
     // basic-state velocity alone; stale_signs: its driver's theta and vapour
     // faces take upwind signs of zero (the sign arrays it never computes)
@@ -116,6 +117,11 @@ __host__ __device__ __forceinline__ int gix(int ny, int nz, int i, int j, int k)
 
 template <typename T>
 __device__ __forceinline__ T sgn(T x) { return x > T(0) ? T(1) : T(-1); }
+// x > 0, in FP64 on the integer pipe: the FP64 pipe (two lanes an SM) bounds
+// the advection.  A positive NaN counts as positive; every use multiplies the
+// result by x.
+__device__ __forceinline__ bool positive(float x) { return x > 0.f; }
+__device__ __forceinline__ bool positive(double x) { return __double_as_longlong(x) > 0; }
 
 // interpolation weights (fluxes.cpp:247-251)
 template <typename T> struct W {
@@ -139,6 +145,12 @@ __device__ __forceinline__ double add_(double a, double b) { return a + b; }
 __device__ __forceinline__ float add_(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ double sub_(double a, double b) { return a - b; }
 __device__ __forceinline__ float sub_(float a, float b) { return __fsub_rn(a, b); }
+
+// the upwind sign of x times 1/60 and 1/12
+template <typename T>
+__device__ __forceinline__ T up60(T x) { return positive(x) ? W<T>::c1_60 : -W<T>::c1_60; }
+template <typename T>
+__device__ __forceinline__ T up12(T x) { return positive(x) ? W<T>::c1_12 : -W<T>::c1_12; }
 
 // INTERP_5TH_EAST (fluxes.cpp:110-122, 155-180): stencil a(-2)..a(+3); cs is
 // the upwind sign times 1/60
@@ -210,30 +222,76 @@ struct Grid {
 
 // six points along i / j around the face between index 0 and +1
 template <typename T>
-__device__ __forceinline__ T f5i(const T *a, const KParams<T> &p, int i, int j, int k, T sign)
+__device__ __forceinline__ T f5i(const T *a, const KParams<T> &p, int i, int j, int k, T cs)
 {
     const int s = p.ny * p.nz, c = gix(p.ny, p.nz, i, j, k);
-    return face5<T>(LD(a, c - 2 * s), LD(a, c - s), LD(a, c), LD(a, c + s), LD(a, c + 2 * s),
-                    LD(a, c + 3 * s), sign);
+    return face5_cs<T>(LD(a, c - 2 * s), LD(a, c - s), LD(a, c), LD(a, c + s), LD(a, c + 2 * s),
+                    LD(a, c + 3 * s), cs);
 }
 template <typename T>
-__device__ __forceinline__ T f5j(const T *a, const KParams<T> &p, int i, int j, int k, T sign)
+__device__ __forceinline__ T f5j(const T *a, const KParams<T> &p, int i, int j, int k, T cs)
 {
     const int s = p.nz, c = gix(p.ny, p.nz, i, j, k);
-    return face5<T>(LD(a, c - 2 * s), LD(a, c - s), LD(a, c), LD(a, c + s), LD(a, c + 2 * s),
-                    LD(a, c + 3 * s), sign);
+    return face5_cs<T>(LD(a, c - 2 * s), LD(a, c - s), LD(a, c), LD(a, c + s), LD(a, c + 2 * s),
+                    LD(a, c + 3 * s), cs);
 }
 template <typename T>
-__device__ __forceinline__ T f3k(const T *a, const KParams<T> &p, int i, int j, int k, T sign)
+__device__ __forceinline__ T f3k(const T *a, const KParams<T> &p, int i, int j, int k, T cs)
 {
     const long c = gix(p.ny, p.nz, i, j, k);
-    return face3<T>(LD(a, c - 1), LD(a, c), LD(a, c + 1), LD(a, c + 2), sign);
+    return face3_cs<T>(LD(a, c - 1), LD(a, c), LD(a, c + 1), LD(a, c + 2), cs);
 }
 template <typename T>
 __device__ __forceinline__ T f2k(const T *a, const KParams<T> &p, int i, int j, int k)
 {
     const long c = gix(p.ny, p.nz, i, j, k);
     return T(0.5) * (LD(a, c + 1) + LD(a, c));
+}
+
+// The faces of a basic state that varies horizontally (field fb: 0 u, 1 v, 2
+// theta, 3 qv; direction 0 east, 1 north, 2 top) depend on the winds through
+// their upwind sign alone, so an FP64 context keeps both values of each face
+// (k_base_faces, built when the basic state is set) and a face costs one load
+// instead of six and 18 operations on the FP64 pipe.
+template <typename T>
+__device__ __forceinline__ const T *bface_at(const KParams<T> &p, int fb, int dir, bool pos)
+{
+    return p.bface + (size_t)((fb * 3 + dir) * 2 + (pos ? 1 : 0)) * p.n;
+}
+template <typename T>
+__device__ __forceinline__ T bar_east(const KParams<T> &p, int fb, const T *b, int i, int j, int k, T x)
+{
+    if (p.bface) return LD(bface_at(p, fb, 0, positive(x)), gix(p.ny, p.nz, i, j, k));
+    return f5i(b, p, i, j, k, up60(x));
+}
+template <typename T>
+__device__ __forceinline__ T bar_north(const KParams<T> &p, int fb, const T *b, int i, int j, int k, T x)
+{
+    if (p.bface) return LD(bface_at(p, fb, 1, positive(x)), gix(p.ny, p.nz, i, j, k));
+    return f5j(b, p, i, j, k, up60(x));
+}
+template <typename T>
+__device__ __forceinline__ T bar_top(const KParams<T> &p, int fb, const T *b, int i, int j, int k, T x)
+{
+    if (p.bface) return LD(bface_at(p, fb, 2, positive(x)), gix(p.ny, p.nz, i, j, k));
+    return f3k(b, p, i, j, k, up12(x));
+}
+template <typename T>
+__global__ void k_base_faces(KParams<T> p, const T *b, int fb, T *out)
+{
+    const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= p.n) return;
+    const int nz = p.nz, k = (int)(t % nz), j = (int)((t / nz) % p.ny), i = (int)(t / ((long)nz * p.ny));
+    if (i < 2 || i > p.nx - 4 || j < 2 || j > p.ny - 4 || k < 1 || k > nz - 2) return;
+    T *o = out + (size_t)fb * 6 * p.n + t;
+    o[0] = f5i(b, p, i, j, k, -W<T>::c1_60);
+    o[p.n] = f5i(b, p, i, j, k, W<T>::c1_60);
+    o[2 * p.n] = f5j(b, p, i, j, k, -W<T>::c1_60);
+    o[3 * p.n] = f5j(b, p, i, j, k, W<T>::c1_60);
+    if (k >= 2 && k <= nz - 3) {
+        o[4 * p.n] = f3k(b, p, i, j, k, -W<T>::c1_12);
+        o[5 * p.n] = f3k(b, p, i, j, k, W<T>::c1_12);
+    }
 }
 
 // the velocity advecting the perturbation at a face: basic state plus
@@ -258,8 +316,8 @@ __device__ T u_east(const KParams<T> &p, const KFields<T> &F, int i, int j, int 
     T ua = T(0.5) * (LD(U, c + s) + LD(U, c));
     T uba = T(0.5) * (LD(UB, c + s) + LD(UB, c));
     const T at = adv_vel(p, uba, ua);
-    T ue = f5i(U, p, i, j, k, sgn(at));
-    T ube = f5i(UB, p, i, j, k, sgn(ua));
+    T ue = f5i(U, p, i, j, k, up60(at));
+    T ube = bar_east(p, 0, UB, i, j, k, ua);
     return flux2(ua, ube, at, ue);
 }
 template <typename T>
@@ -270,8 +328,8 @@ __device__ T u_north(const KParams<T> &p, const KFields<T> &F, int i, int j, int
     T va = T(0.5) * (LD(V, a) + LD(V, b));
     T vba = T(0.5) * (LD(VB, a) + LD(VB, b));
     const T at = adv_vel(p, vba, va);
-    T un = f5j(U, p, i, j, k, sgn(at));
-    T ubn = f5j(UB, p, i, j, k, sgn(va));
+    T un = f5j(U, p, i, j, k, up60(at));
+    T ubn = bar_north(p, 0, UB, i, j, k, va);
     return flux2(va, ubn, at, un);
 }
 template <typename T>
@@ -287,8 +345,8 @@ __device__ T u_top(const KParams<T> &p, const KFields<T> &F, int i, int j, int k
         ut = f2k(U, p, i, j, k);
         ubt = f2k(UB, p, i, j, k);
     } else {
-        ut = f3k(U, p, i, j, k, sgn(adv_vel(p, wba, wa)));
-        ubt = f3k(UB, p, i, j, k, sgn(wa));
+        ut = f3k(U, p, i, j, k, up12(adv_vel(p, wba, wa)));
+        ubt = bar_top(p, 0, UB, i, j, k, wa);
     }
     return flux2(wa, ubt, adv_vel(p, wba, wa), ut);
 }
@@ -300,8 +358,8 @@ __device__ T v_east(const KParams<T> &p, const KFields<T> &F, int i, int j, int 
     T ua = T(0.5) * (LD(U, a) + LD(U, b));
     T uba = T(0.5) * (LD(UB, a) + LD(UB, b));
     const T at = adv_vel(p, uba, ua);
-    T ve = f5i(V, p, i, j, k, sgn(at));
-    T vbe = f5i(VB, p, i, j, k, sgn(ua));
+    T ve = f5i(V, p, i, j, k, up60(at));
+    T vbe = bar_east(p, 1, VB, i, j, k, ua);
     return flux2(ua, vbe, at, ve);
 }
 template <typename T>
@@ -312,8 +370,8 @@ __device__ T v_north(const KParams<T> &p, const KFields<T> &F, int i, int j, int
     T va = T(0.5) * (LD(V, c + p.nz) + LD(V, c));
     T vba = T(0.5) * (LD(VB, c + p.nz) + LD(VB, c));
     const T at = adv_vel(p, vba, va);
-    T vn = f5j(V, p, i, j, k, sgn(at));
-    T vbn = f5j(VB, p, i, j, k, sgn(va));
+    T vn = f5j(V, p, i, j, k, up60(at));
+    T vbn = bar_north(p, 1, VB, i, j, k, va);
     return flux2(va, vbn, at, vn);
 }
 template <typename T>
@@ -329,8 +387,8 @@ __device__ T v_top(const KParams<T> &p, const KFields<T> &F, int i, int j, int k
         vt = f2k(V, p, i, j, k);
         vbt = f2k(VB, p, i, j, k);
     } else {
-        vt = f3k(V, p, i, j, k, sgn(adv_vel(p, wba, wa)));
-        vbt = f3k(VB, p, i, j, k, sgn(wa));
+        vt = f3k(V, p, i, j, k, up12(adv_vel(p, wba, wa)));
+        vbt = bar_top(p, 1, VB, i, j, k, wa);
     }
     return flux2(wa, vbt, adv_vel(p, wba, wa), vt);
 }
@@ -349,9 +407,10 @@ __device__ T s_east(const KParams<T> &p, const KFields<T> &F, const T *s, const 
     // the linearised driver's stale signs, except on the face east of column
     // 2, which compute_west_scalar (fluxes.cpp:479-501) forms from the winds
     const bool z = sb && p.stale_signs && i != 2;
-    T se = f5i(s, p, i, j, k, z ? T(0) : sgn(ut));
+    T se = f5i(s, p, i, j, k, z ? T(0) : up60(ut));
     if (!sb) return ut * se;
-    T be = f5i(sb, p, i, j, k, z ? T(0) : sgn(u1));
+    const int fb = sb == F.bar[3] ? 2 : 3;
+    T be = z ? f5i(sb, p, i, j, k, T(0)) : bar_east(p, fb, sb, i, j, k, u1);
     return flux2(u1, be, ut, se);
 }
 template <typename T>
@@ -361,9 +420,10 @@ __device__ T s_north(const KParams<T> &p, const KFields<T> &F, const T *s, const
     T v1 = LD(F.cur[FV], a);
     T vt = sb ? adv_vel(p, LD(F.bar[1], a), v1) : LD(F.bar[1], a) + v1;
     const bool z = sb && p.stale_signs;
-    T sn = f5j(s, p, i, j, k, z ? T(0) : sgn(vt));
+    T sn = f5j(s, p, i, j, k, z ? T(0) : up60(vt));
     if (!sb) return vt * sn;
-    T bn = f5j(sb, p, i, j, k, z ? T(0) : sgn(v1));
+    const int fb = sb == F.bar[3] ? 2 : 3;
+    T bn = z ? f5j(sb, p, i, j, k, T(0)) : bar_north(p, fb, sb, i, j, k, v1);
     return flux2(v1, bn, vt, sn);
 }
 template <typename T>
@@ -379,8 +439,8 @@ __device__ T s_top(const KParams<T> &p, const KFields<T> &F, const T *s, const T
         if (sb) bt = f2k(sb, p, i, j, k);
     } else {
         const bool z = sb && p.stale_signs;
-        st = f3k(s, p, i, j, k, z ? T(0) : sgn(wt));
-        if (sb) bt = f3k(sb, p, i, j, k, z ? T(0) : sgn(w1));
+        st = f3k(s, p, i, j, k, z ? T(0) : up12(wt));
+        if (sb) bt = z ? f3k(sb, p, i, j, k, T(0)) : bar_top(p, sb == F.bar[3] ? 2 : 3, sb, i, j, k, w1);
     }
     if (!sb) return wt * st;
     return flux2(w1, bt, wt, st);
@@ -427,7 +487,7 @@ __device__ T r_top(const KParams<T> &p, const KFields<T> &F, int i, int j, int k
     T wf = wb - T(0.5) * (vt_at(p, F, i, j, k) + vt_at(p, F, i, j, k + 1));
     T st;
     if (k == 1 || k == p.nz - 2) st = f2k(s, p, i, j, k);
-    else st = f3k(s, p, i, j, k, sgn(wf));
+    else st = f3k(s, p, i, j, k, up12(wf));
     return wf * st;
 }
 
@@ -582,9 +642,9 @@ __global__ void k_base_tables(KParams<T> p, const T *ub, const T *vb, const T *w
 #define BTAB(row, k) p.btab[(row) * p.nz + (k)]
 
 template <typename T>
-__device__ __forceinline__ T face3_tab(const KParams<T> &p, int rc4, int k, T sign)
+__device__ __forceinline__ T face3_tab(const KParams<T> &p, int rc4, int k, T cs)
 {
-    return fma_(mul_(W<T>::c1_12, sign), BTAB(rc4 + 1, k), BTAB(rc4, k));
+    return fma_(cs, BTAB(rc4 + 1, k), BTAB(rc4, k));
 }
 
 template <typename T>
@@ -594,7 +654,7 @@ __device__ T u_east_ub(const KParams<T> &p, const KFields<T> &F, int i, int j, i
     const int c = gix(p.ny, p.nz, i, j, k), s = p.ny * p.nz;
     T ua = T(0.5) * (LD(U, c + s) + LD(U, c));
     T uba = BTAB(BT_UA, k);
-    T ue = f5i(U, p, i, j, k, sgn(uba + ua));
+    T ue = f5i(U, p, i, j, k, up60(uba + ua));
     return flux2(ua, BTAB(BT_C6_UB, k), (uba + ua), ue);
 }
 template <typename T>
@@ -604,7 +664,7 @@ __device__ T u_north_ub(const KParams<T> &p, const KFields<T> &F, int i, int j, 
     const int a = gix(p.ny, p.nz, i, j + 1, k), b = gix(p.ny, p.nz, i - 1, j + 1, k);
     T va = T(0.5) * (LD(V, a) + LD(V, b));
     T vba = BTAB(BT_VA, k);
-    T un = f5j(U, p, i, j, k, sgn(vba + va));
+    T un = f5j(U, p, i, j, k, up60(vba + va));
     return flux2(va, BTAB(BT_C6_UB, k), (vba + va), un);
 }
 template <typename T>
@@ -620,8 +680,8 @@ __device__ T u_top_ub(const KParams<T> &p, const KFields<T> &F, int i, int j, in
         ut = f2k(U, p, i, j, k);
         ubt = BTAB(BT_H2_UB, k);
     } else {
-        ut = f3k(U, p, i, j, k, sgn(wba + wa));
-        ubt = face3_tab(p, BT_C4_UB, k, sgn(wa));
+        ut = f3k(U, p, i, j, k, up12(wba + wa));
+        ubt = face3_tab(p, BT_C4_UB, k, up12(wa));
     }
     return flux2(wa, ubt, wba + wa, ut);
 }
@@ -632,7 +692,7 @@ __device__ T v_east_ub(const KParams<T> &p, const KFields<T> &F, int i, int j, i
     const int a = gix(p.ny, p.nz, i + 1, j, k), b = gix(p.ny, p.nz, i + 1, j - 1, k);
     T ua = T(0.5) * (LD(U, a) + LD(U, b));
     T uba = BTAB(BT_UA, k);
-    T ve = f5i(V, p, i, j, k, sgn(uba + ua));
+    T ve = f5i(V, p, i, j, k, up60(uba + ua));
     return flux2(ua, BTAB(BT_C6_VB, k), (uba + ua), ve);
 }
 template <typename T>
@@ -642,7 +702,7 @@ __device__ T v_north_ub(const KParams<T> &p, const KFields<T> &F, int i, int j, 
     const int c = gix(p.ny, p.nz, i, j, k);
     T va = T(0.5) * (LD(V, c + p.nz) + LD(V, c));
     T vba = BTAB(BT_VA, k);
-    T vn = f5j(V, p, i, j, k, sgn(vba + va));
+    T vn = f5j(V, p, i, j, k, up60(vba + va));
     return flux2(va, BTAB(BT_C6_VB, k), (vba + va), vn);
 }
 template <typename T>
@@ -658,8 +718,8 @@ __device__ T v_top_ub(const KParams<T> &p, const KFields<T> &F, int i, int j, in
         vt = f2k(V, p, i, j, k);
         vbt = BTAB(BT_H2_VB, k);
     } else {
-        vt = f3k(V, p, i, j, k, sgn(wba + wa));
-        vbt = face3_tab(p, BT_C4_VB, k, sgn(wa));
+        vt = f3k(V, p, i, j, k, up12(wba + wa));
+        vbt = face3_tab(p, BT_C4_VB, k, up12(wa));
     }
     return flux2(wa, vbt, wba + wa, vt);
 }
@@ -670,7 +730,7 @@ __device__ T s_east_ub(const KParams<T> &p, const KFields<T> &F, const T *s, int
     const int a = gix(p.ny, p.nz, i + 1, j, k);
     T u1 = LD(F.cur[FU], a);
     T ut = BTAB(BT_UB, k) + u1;
-    T se = f5i(s, p, i, j, k, sgn(ut));
+    T se = f5i(s, p, i, j, k, up60(ut));
     if (brow < 0) return ut * se;
     return flux2(u1, BTAB(BT_C6_THB + brow, k), ut, se);
 }
@@ -680,7 +740,7 @@ __device__ T s_north_ub(const KParams<T> &p, const KFields<T> &F, const T *s, in
     const int a = gix(p.ny, p.nz, i, j + 1, k);
     T v1 = LD(F.cur[FV], a);
     T vt = BTAB(BT_VB, k) + v1;
-    T sn = f5j(s, p, i, j, k, sgn(vt));
+    T sn = f5j(s, p, i, j, k, up60(vt));
     if (brow < 0) return vt * sn;
     return flux2(v1, BTAB(BT_C6_THB + brow, k), vt, sn);
 }
@@ -696,8 +756,8 @@ __device__ T s_top_ub(const KParams<T> &p, const KFields<T> &F, const T *s, int 
         st = f2k(s, p, i, j, k);
         if (brow >= 0) bt = BTAB(BT_H2_THB + brow, k);
     } else {
-        st = f3k(s, p, i, j, k, sgn(wt));
-        if (brow >= 0) bt = face3_tab(p, BT_C4_THB + 2 * brow, k, sgn(w1));
+        st = f3k(s, p, i, j, k, up12(wt));
+        if (brow >= 0) bt = face3_tab(p, BT_C4_THB + 2 * brow, k, up12(w1));
     }
     if (brow < 0) return wt * st;
     return flux2(w1, bt, wt, st);
@@ -715,7 +775,7 @@ __device__ T r_top_ub(const KParams<T> &p, const KFields<T> &F, int i, int j, in
     T wf = wb - T(0.5) * (vt_at(p, F, i, j, k) + vt_at(p, F, i, j, k + 1));
     T st;
     if (k == 1 || k == p.nz - 2) st = f2k(s, p, i, j, k);
-    else st = f3k(s, p, i, j, k, sgn(wf));
+    else st = f3k(s, p, i, j, k, up12(wf));
     return wf * st;
 }
 
@@ -813,11 +873,31 @@ __device__ __forceinline__ void faces_top(const KParams<T> &p, const KFields<T> 
     }
 }
 
+// threads of a tile block: FP64 tiles keep the FP64 pipe busier with twice as
+// many warps (at 256 threads and one block an SM it was active 78% of the time)
+constexpr int ADV_MAXT = 512;
+template <typename T> __host__ __device__ constexpr int adv_threads() { return sizeof(T) == 8 ? 512 : 256; }
+// flux fields of a launch, and its shared memory: their face stores and the
+// buoyancy columns (all six fields where the launch is not known)
+__host__ __device__ constexpr int advect_tile_fields(int what)
+{
+    return ((what & ADV_UV) ? 2 : 0) + ((what & ADV_TH) ? 1 : 0) + ((what & ADV_Q) ? 3 : 0);
+}
+__host__ __device__ constexpr size_t advect_tile_smem(int ti, int tj, int nz, size_t tsize,
+                                                      int what = ADV_UV | ADV_TH | ADV_Q)
+{
+    return ((size_t)advect_tile_fields(what) * ((ti + 1) * tj + ti * (tj + 1) + ti * tj) +
+            ((what & ADV_WB) ? ti * tj : 0)) *
+           nz * tsize;
+}
+
 template <typename T, int TI = ADV_TI, int TJ = ADV_TJ>
 __device__ void advect_tile_body(const KParams<T> &p, const KFields<T> &F, int bx, int by, T step, T sdtg, int what)
 {
     extern __shared__ unsigned char smem_raw[];
-    const int NF = ADV_NF;
+    const int NF = advect_tile_fields(what);
+    // store slots of the launch's flux fields: u, v; theta; qv, qc, qr
+    const int s_th = (what & ADV_UV) ? 2 : 0, s_q = s_th + ((what & ADV_TH) ? 1 : 0);
     const int nz = p.nz, nzi = nz - 2;
     const int i0 = 3 + bx * TI, j0 = 3 + by * TJ;
     const int ti = min(TI, p.nx - 3 - i0), tj = min(TJ, p.ny - 3 - j0);
@@ -825,16 +905,28 @@ __device__ void advect_tile_body(const KParams<T> &p, const KFields<T> &F, int b
     T *E = (T *)smem_raw;                    // [(TI+1)][TJ] columns, east face of column i0-1+a
     T *Nf = E + NF * (TI + 1) * TJ * nz;      // [TI][(TJ+1)] columns, north face of column j0-1+b
     T *Tf = Nf + NF * TI * (TJ + 1) * nz;     // [TI][TJ] columns, top face at level k
+    T *Bf = Tf + NF * TI * TJ * nz;           // [TI][TJ] columns, buoyancy at level k
     const int sE = (TI + 1) * TJ * nz, sN = TI * (TJ + 1) * nz, sT = TI * TJ * nz;
-    T tmp[NF];
+    T tmp[ADV_NF];
+    auto put = [&](T *dst, int stride) {
+        if (what & ADV_UV) {
+            dst[0] = tmp[0];
+            dst[stride] = tmp[1];
+        }
+        if (what & ADV_TH) dst[s_th * stride] = tmp[2];
+        if (what & ADV_Q) {
+            dst[s_q * stride] = tmp[3];
+            dst[(s_q + 1) * stride] = tmp[4];
+            dst[(s_q + 2) * stride] = tmp[5];
+        }
+    };
     // phase 1a: east faces of columns i0-1 .. i0+ti-1
     for (int w = threadIdx.x; w < (TI + 1) * TJ * nzi; w += blockDim.x) {
         const int kk = w % nzi, c = w / nzi, b = c % TJ, a = c / TJ;
         if (a > ti || b >= tj) continue;
         faces_east(p, F, what, i0 - 1 + a, j0 + b, 1 + kk, tmp);
         const int o = (a * TJ + b) * nz + 1 + kk;
-#pragma unroll
-        for (int f = 0; f < NF; f++) E[f * sE + o] = tmp[f];
+        put(E + o, sE);
     }
     // phase 1b: north faces of rows j0-1 .. j0+tj-1
     for (int w = threadIdx.x; w < TI * (TJ + 1) * nzi; w += blockDim.x) {
@@ -842,8 +934,7 @@ __device__ void advect_tile_body(const KParams<T> &p, const KFields<T> &F, int b
         if (a >= ti || b > tj) continue;
         faces_north(p, F, what, i0 + a, j0 - 1 + b, 1 + kk, tmp);
         const int o = (a * (TJ + 1) + b) * nz + 1 + kk;
-#pragma unroll
-        for (int f = 0; f < NF; f++) Nf[f * sN + o] = tmp[f];
+        put(Nf + o, sN);
     }
     // phase 1c: top faces at levels 0 .. nz-2
     for (int w = threadIdx.x; w < TI * TJ * (nz - 1); w += blockDim.x) {
@@ -851,8 +942,19 @@ __device__ void advect_tile_body(const KParams<T> &p, const KFields<T> &F, int b
         if (a >= ti || b >= tj) continue;
         faces_top(p, F, what, i0 + a, j0 + b, k, tmp);
         const int o = (a * TJ + b) * nz + k;
-#pragma unroll
-        for (int f = 0; f < NF; f++) Tf[f * sT + o] = tmp[f];
+        put(Tf + o, sT);
+        if ((what & ADV_WB) && k >= 1) {  // buoyancy of the level, used by its own and the next one's w
+            const int cix = gix(p.ny, nz, i0 + a, j0 + b, k);
+            T bk;
+            if (!p.moist) {
+                bk = LD(F.cur[FTH], cix) / p.tbv[k];
+            } else {
+                bk = buoy_moist(LD(F.cur[FTH], cix), p.tbv[k], LD(F.cur[FQV], cix), LD(F.cur[FQC], cix),
+                                LD(F.cur[FQR], cix));
+                if (p.ice) bk = bk - LD(F.cur[FQI], cix) - LD(F.cur[FQS], cix);  // buoyancy_cold_micro (advection.cpp:56-58)
+            }
+            Bf[o] = bk;
+        }
     }
     __syncthreads();
     // phase 2: tendencies
@@ -879,27 +981,11 @@ __device__ void advect_tile_body(const KParams<T> &p, const KFields<T> &F, int b
             const T vt = fma_(-mul_(p.dt, p.f[j]), ov_v, tend(1));
             F.P[FV][cix] = fma_(step, vt, LD(F.M[FV], cix));
         }
-        if ((what & ADV_WB) && k >= 2) {
-            const T *TH = F.cur[FTH];
-            T b0, b1;
-            if (!p.moist) {
-                b0 = LD(TH, cix) / p.tbv[k];
-                b1 = LD(TH, cix - 1) / p.tbv[k - 1];
-            } else {
-                const T *QV = F.cur[FQV], *QC = F.cur[FQC], *QR = F.cur[FQR];
-                b0 = buoy_moist(LD(TH, cix), p.tbv[k], LD(QV, cix), LD(QC, cix), LD(QR, cix));
-                b1 = buoy_moist(LD(TH, cix - 1), p.tbv[k - 1], LD(QV, cix - 1), LD(QC, cix - 1), LD(QR, cix - 1));
-                if (p.ice) {  // buoyancy_cold_micro (advection.cpp:56-58)
-                    const T *QI = F.cur[FQI], *QS = F.cur[FQS];
-                    b0 = b0 - LD(QI, cix) - LD(QS, cix);
-                    b1 = b1 - LD(QI, cix - 1) - LD(QS, cix - 1);
-                }
-            }
-            F.P[FW][cix] = fma_(sdtg, add_(b0, b1), LD(F.M[FW], cix));
-        }
+        if ((what & ADV_WB) && k >= 2)
+            F.P[FW][cix] = fma_(sdtg, add_(Bf[ot], Bf[ot - 1]), LD(F.M[FW], cix));
         const T *Wc = F.cur[FW];
         if (what & ADV_TH) {
-            const T t = sub_base(tend(2), DTZ, p.rhow[k + 1], LD(Wc, cix + 1), p.tb[k + 1] - p.tb[k], p.rhow[k],
+            const T t = sub_base(tend(s_th), DTZ, p.rhow[k + 1], LD(Wc, cix + 1), p.tb[k + 1] - p.tb[k], p.rhow[k],
                                  LD(Wc, cix), p.tb[k] - p.tb[k - 1], p.one_d_rhou[k]);
             F.P[FTH][cix] = fma_(step, t, LD(F.M[FTH], cix));
         }
@@ -909,11 +995,11 @@ __device__ void advect_tile_body(const KParams<T> &p, const KFields<T> &F, int b
                 F.vt[cix] = fall_speed_point(p, LD(QR, cix), k);
                 if (k == 1) F.vt[cix - 1] = fall_speed_point(p, LD(QR, cix), 1);
             }
-            const T tv = sub_base(tend(3), DTZ, p.rhow[k + 1], LD(Wc, cix + 1), p.qb[k + 1] - p.qb[k], p.rhow[k],
+            const T tv = sub_base(tend(s_q), DTZ, p.rhow[k + 1], LD(Wc, cix + 1), p.qb[k + 1] - p.qb[k], p.rhow[k],
                                   LD(Wc, cix), p.qb[k] - p.qb[k - 1], p.one_d_rhou[k]);
             T qv = fma_(step, tv, LD(F.M[FQV], cix));
-            T qc = fma_(step, tend(4), LD(F.M[FQC], cix));
-            T qr = fma_(step, tend(5), LD(F.M[FQR], cix));
+            T qc = fma_(step, tend(s_q + 1), LD(F.M[FQC], cix));
+            T qr = fma_(step, tend(s_q + 2), LD(F.M[FQR], cix));
             if (what & ADV_ZERO) {
                 unsigned char bits = 0;
                 if (qc < 0) { qc = 0; bits |= 2; }
@@ -932,15 +1018,9 @@ __device__ void advect_tile_body(const KParams<T> &p, const KFields<T> &F, int b
 }
 
 template <typename T, int TI = ADV_TI, int TJ = ADV_TJ>
-__global__ void __launch_bounds__(256) k_advect_tile(KParams<T> p, KFields<T> F, T step, T sdtg, int what)
+__global__ void __launch_bounds__(ADV_MAXT, 1) k_advect_tile(KParams<T> p, KFields<T> F, T step, T sdtg, int what)
 {
     advect_tile_body<T, TI, TJ>(p, F, blockIdx.x, blockIdx.y, step, sdtg, what);
-}
-
-// shared memory of an advection tile: the face stores of every flux field
-__host__ __device__ constexpr size_t advect_tile_smem(int ti, int tj, int nz, size_t tsize)
-{
-    return (size_t)ADV_NF * ((ti + 1) * tj + ti * (tj + 1) + ti * tj) * nz * tsize;
 }
 
 // ---------------------------------------------------------------------------

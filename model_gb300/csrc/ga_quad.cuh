@@ -972,6 +972,11 @@ __device__ __forceinline__ void stv(double *a, const LV<double> &q)
     *reinterpret_cast<double2 *>(a) = make_double2(q.v[0], q.v[1]);
 }
 
+// Keeps a branch a branch: the sponge strips and the damping levels are few,
+// and evaluated everywhere under selects they were two thirds of the FP64
+// pass's operations on the FP64 pipe.
+__device__ __forceinline__ void rare_path() { asm volatile(""); }
+
 // item w: column w / (NZ/4) of the enumeration `cols`, level quad w % (NZ/4).
 // KES: the step's last pass with Kessler (run_kessler_microphysics,
 // kessler.cpp:25-213) and the Eulerian precipitation (precip_rate,
@@ -1006,6 +1011,7 @@ __device__ __forceinline__ void post_quad_body(const KParams<T> &p, const KField
     const bool hN = si >= 1 && j >= p.nb && j < p.ne;
     const T cE = hE ? p.ce[si - p.eb] : T(0), cW = hW ? p.cw[si - p.wb] : T(0);
     const T cS = hS ? p.cs[j - p.sb] : T(0), cN = hN ? p.cn[j - p.nb] : T(0);
+    const bool strip = hE || hW || hS || hN;
     T dpx[L] = {}, dpy[L] = {}, dpz[L] = {};
     if (col_in && ((flv[FU] | flv[FV] | flv[FW]) & PF_PROJECT)) {
         const LV<T> pc = ldv(F.pi + cs), px = ldv(F.pi + cs - sx), py = ldv(F.pi + cs - sy);
@@ -1073,7 +1079,8 @@ __device__ __forceinline__ void post_quad_body(const KParams<T> &p, const KField
                 else if (f == FV) v = v - step * (p.dty * dpy[e]);
                 else if (f == FW && k >= 2) v = v - step * ((p.dtz * p.mw[k]) * dpz[e]);
             }
-            if ((flags & PF_SPONGE) && k >= 1) {
+            if ((flags & PF_SPONGE) && strip && k >= 1) {
+                rare_path();
                 if (hE) v = v - cE * v;
                 if (hW) v = v - cW * v;
                 if (hS) v = v - cS * v;
@@ -1095,6 +1102,7 @@ __device__ __forceinline__ void post_quad_body(const KParams<T> &p, const KField
                 }
             }
             if ((flags & PF_RAYLEIGH) && f <= FTH && ray_col && k >= p.raylevel) {  // damping.cpp:1148-1177
+                rare_path();
                 const T cr = (f == FW) ? p.ray_w[k] : p.ray_u[k];
                 v = v - cr * v;
             }
