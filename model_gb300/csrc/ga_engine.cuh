@@ -1312,9 +1312,9 @@ class Engine : public EngineBase {
             const long tv = (long)(NX - 2) * (NY - 2) * NZ;
             k_fall_speed<T><<<cdiv(tv, 256), 256, 0, stream>>>(kp, F);
             const long ncol = (long)(NX - 2) * (NY - 2);
-            k_ppm_prepare<T><<<cdiv(ncol, 64), 64, 0, stream>>>(kp, F, ppm_has, ppm_topq, ppm_topm);
-            k_ppm_carry<T><<<1, 32, 0, stream>>>(ncol, ppm_has, ppm_topq, ppm_topm, ppm_cin, ppm_carry);
-            k_ppm_remap<T><<<cdiv(ncol, 64), 64, 0, stream>>>(kp, F, ppm_has, ppm_cin);
+            k_ppm_prepare<T><<<cdiv(ncol, PPM_WARPS), 32 * PPM_WARPS, 0, stream>>>(kp, F, ppm_has, ppm_topq, ppm_topm);
+            k_ppm_carry<T><<<1, PPM_CARRY, 0, stream>>>(ncol, ppm_has, ppm_topq, ppm_topm, ppm_cin, ppm_carry);
+            k_ppm_remap<T><<<cdiv(ncol, PPM_WARPS), 32 * PPM_WARPS, 0, stream>>>(kp, F, ppm_has, ppm_cin);
             k_fill<T><<<cdiv(N, 256), 256, 0, stream>>>(vt, N, T(0));
             launches += 5;
         }
@@ -1349,9 +1349,9 @@ class Engine : public EngineBase {
         F.vt = fall;
         F.accrain = acc;
         const long ncol = (long)(NX - 2) * (NY - 2);
-        k_ppm_prepare<T><<<cdiv(ncol, 64), 64, 0, stream>>>(kp, F, ppm_has, ppm_topq, ppm_topm);
-        k_ppm_carry<T><<<1, 32, 0, stream>>>(ncol, ppm_has, ppm_topq, ppm_topm, ppm_cin, ppm_carry);
-        k_ppm_remap<T><<<cdiv(ncol, 64), 64, 0, stream>>>(kp, F, ppm_has, ppm_cin);
+        k_ppm_prepare<T><<<cdiv(ncol, PPM_WARPS), 32 * PPM_WARPS, 0, stream>>>(kp, F, ppm_has, ppm_topq, ppm_topm);
+        k_ppm_carry<T><<<1, PPM_CARRY, 0, stream>>>(ncol, ppm_has, ppm_topq, ppm_topm, ppm_cin, ppm_carry);
+        k_ppm_remap<T><<<cdiv(ncol, PPM_WARPS), 32 * PPM_WARPS, 0, stream>>>(kp, F, ppm_has, ppm_cin);
         launches += 3;
     }
 
