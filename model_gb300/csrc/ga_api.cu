@@ -205,9 +205,7 @@ int ga_step(ga_ctx *ctx, int nsteps)
 {
     int rc = ga_step_async(ctx, nsteps);
     if (rc) return rc;
-    rc = ga_synchronize(ctx);
-    if (rc) return rc;
-    return ctx->e->op(GA_OP_SIGN_CELLS, 0.0);  /* reports a Kessler E>100 flag */
+    return ctx->e->step_status();  /* reports a Kessler E>100 flag */
 }
 
 int ga_op(ga_ctx *ctx, int op, double step)

@@ -54,6 +54,7 @@ class Engine : public EngineBase {
     std::vector<void *> allocs;
     KParams<T> kp;
     int *d_err = nullptr;
+    int *h_err = nullptr;  // pinned copy of d_err, made by sync_status
     unsigned char *ppm_has = nullptr;
     T *ppm_topq = nullptr, *ppm_topm = nullptr, *ppm_cin = nullptr, *ppm_carry = nullptr;
     double *staging = nullptr;
@@ -76,6 +77,7 @@ class Engine : public EngineBase {
     int status = GA_OK;
     std::unique_ptr<LinBase> lin;  // tangent-linear / adjoint buffers, on first use
     int adv_ti = ADV_TI, adv_tj = ADV_TJ;  // advection tile (autotuned)
+    bool adv_tuned = false;
     // the four-level advection kernel (FP32, uniform basic state, NZ % 4 == 0)
     // and its tile; GA_ADVECT=tile or =quad restricts both the default and the
     // autotuner to one kernel
@@ -299,6 +301,8 @@ class Engine : public EngineBase {
         vt = dalloc<T>(N);
         accrain = dalloc<double>((size_t)NX * NY);
         d_err = dalloc<int>(2);  // [0] Kessler, [1] staging (kErrStaging)
+        if (cudaMallocHost(&h_err, 2 * sizeof(int)) != cudaSuccess) { status = GA_ERR_NOMEM; return; }
+        h_err[0] = h_err[1] = 0;
         const int periodic = c->periodic_ew_boundaries;
         const int ni = periodic ? NX - 6 : NX, nj = NY;
         const int nh = spec_nh(nj), nzs = spec_nzs(NZ);
@@ -629,6 +633,7 @@ class Engine : public EngineBase {
         for (void *p : allocs) cudaFree(p);
         if (staging) cudaFree(staging);
         if (bface) cudaFree(bface);
+        if (h_err) cudaFreeHost(h_err);
         if (stream2) cudaStreamSynchronize(stream2);
         if (ev_fork) cudaEventDestroy(ev_fork);
         if (ev_join) cudaEventDestroy(ev_join);
@@ -798,8 +803,10 @@ class Engine : public EngineBase {
         return sync_status();
     }
 
+    // waits for the stream; the error words come back in the same wait
     int sync_status()
     {
+        cudaMemcpyAsync(h_err, d_err, 2 * sizeof(int), cudaMemcpyDeviceToHost, stream);
         cudaError_t e = cudaStreamSynchronize(stream);
         if (e != cudaSuccess) {
             set_error(std::string("CUDA: ") + cudaGetErrorString(e));
@@ -1006,9 +1013,7 @@ class Engine : public EngineBase {
     // the staging bit of the device error word (a bounded wait ran out)
     int staging_status()
     {
-        int e = 0;
-        cudaMemcpy(&e, d_err + 1, sizeof(int), cudaMemcpyDeviceToHost);
-        if (e & kErrStaging) {
+        if (h_err[1] & kErrStaging) {
             set_error("advection: a shared-memory staging copy did not complete within its bound");
             return GA_ERR_CUDA;
         }
@@ -1151,7 +1156,13 @@ class Engine : public EngineBase {
             else launch_advect_quad<4, 8>(st, sg, wq);
         } else if (smem_adv <= 200 * 1024) {
             const T st = (T)step, sg = (T)sdtg;
-            if (adv_ti == 2) launch_advect_tile<2, 4>(st, sg, what);
+            // FP64, untuned: the 4x8 tile's fewer shared faces (3.4 a cell
+            // against 3.5) where two blocks of it fit an SM (192x128x32, dry:
+            // 0.457 against 0.477 ms); with six fields' faces only one does
+            const bool wide = sizeof(T) == 8 && adv_ti == ADV_TI && adv_tj == ADV_TJ && !adv_tuned &&
+                              advect_tile_smem(4, 8, NZ, sizeof(T), what) <= 110 * 1024;
+            if (wide) launch_advect_tile<4, 8>(st, sg, what);
+            else if (adv_ti == 2) launch_advect_tile<2, 4>(st, sg, what);
             else if (adv_tj == 2) launch_advect_tile<4, 2>(st, sg, what);
             else if (adv_tj == 8) launch_advect_tile<4, 8>(st, sg, what);
             else if (adv_ti == 8) launch_advect_tile<8, 4>(st, sg, what);
@@ -1503,12 +1514,19 @@ class Engine : public EngineBase {
         }
         // a captured two-step graph pairs the rotation parity with the
         // diffusion buffers' parity; a single operator may break the pairing
-        if (diff_tend) drop_graphs();
+        if (diff_tend && o != GA_OP_SIGN_CELLS) drop_graphs();
         int rc = launch_status();
         if (rc) return rc;
         rc = sync_status();
         if (rc) return rc;
         return kessler_status();
+    }
+
+    int step_status() override
+    {
+        cudaSetDevice(device);
+        const int rc = sync_status();
+        return rc ? rc : kessler_status();
     }
 
     void periodic_pi()
@@ -1521,9 +1539,7 @@ class Engine : public EngineBase {
     int kessler_status()
     {
         if (!kp.moist) return GA_OK;
-        int e = 0;
-        cudaMemcpy(&e, d_err, sizeof(int), cudaMemcpyDeviceToHost);
-        if (e) {
+        if (h_err[0]) {
             set_error(kp.ice ? "ice microphysics: rain evaporation E>100 or snow melting |psmlt|>100 (the reference "
                                "exits here, rutledge.cpp:252-258, 370-376)"
                              : "Kessler evaporation E>100 (the reference exits here, kessler.cpp:83-88)");
@@ -1832,6 +1848,7 @@ class Engine : public EngineBase {
                           g.tj, best);
             info += line;
         } else {  // advection tile
+            adv_tuned = true;
             float best = 1e30f;
             int bi = adv_ti, bj = adv_tj, bq = 0, qi = adv_qi, qj = adv_qj, qb = adv_qb, br = adv_rows;
             int bt = 0, tc = adv_tmc;

@@ -34,6 +34,7 @@ struct EngineBase {
     virtual int get_field(int field, int slot, double *host, size_t n) = 0;
     virtual int op(int op, double step) = 0;
     virtual int step(int nsteps) = 0;
+    virtual int step_status() = 0;  // waits for queued steps; CUDA and Kessler errors
     virtual int check_finite() = 0;
     virtual int budget(int slot, double *out) = 0;  // GA_NBUDGET FP64 domain sums
     virtual void *field_ptr(int field, int slot) = 0;

@@ -875,7 +875,6 @@ __device__ __forceinline__ void faces_top(const KParams<T> &p, const KFields<T> 
 
 // threads of a tile block: FP64 tiles keep the FP64 pipe busier with twice as
 // many warps (at 256 threads and one block an SM it was active 78% of the time)
-constexpr int ADV_MAXT = 512;
 template <typename T> __host__ __device__ constexpr int adv_threads() { return sizeof(T) == 8 ? 512 : 256; }
 // flux fields of a launch, and its shared memory: their face stores and the
 // buoyancy columns (all six fields where the launch is not known)
@@ -1018,7 +1017,7 @@ __device__ void advect_tile_body(const KParams<T> &p, const KFields<T> &F, int b
 }
 
 template <typename T, int TI = ADV_TI, int TJ = ADV_TJ>
-__global__ void __launch_bounds__(ADV_MAXT, 1) k_advect_tile(KParams<T> p, KFields<T> F, T step, T sdtg, int what)
+__global__ void __launch_bounds__(adv_threads<T>(), sizeof(T) == 8 ? 2 : 4) k_advect_tile(KParams<T> p, KFields<T> F, T step, T sdtg, int what)
 {
     advect_tile_body<T, TI, TJ>(p, F, blockIdx.x, blockIdx.y, step, sdtg, what);
 }
