@@ -431,10 +431,11 @@ class Engine : public EngineBase {
             hyd.pf = col_T(pf.data(), (int)pf.size());
             hyd.rden = col_T(rden.data(), (int)rden.size());
             hyd.ac = col_T(ac.data(), NY);
-            hyd.pw = dalloc<T>((size_t)NX * 2 * (NY + 1));
             hyd.div = dalloc<T>((size_t)NX * NY);
             hyd.spec2 = dalloc<T2>((size_t)NX * NY);
-            hyd_L = (int)std::max<size_t>(1, std::min<size_t>(8, 49152 / (2 * (size_t)NX * sizeof(T2))));
+            if (hyd_thomas_smem<T>(NY) > 200 * 1024) hyd.tw = dalloc<T>((size_t)cdiv(NX, HT) * HT * NY * 4);
+            cudaFuncSetAttribute(k_hyd_thomas<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+            hyd_L = (int)std::max<size_t>(1, std::min<size_t>(4, 49152 / (2 * (size_t)NX * sizeof(T2))));
         }
         if (c->linear_model) {  // linear_integrate_rk3: eager steps (a rescaling may fall on any step)
             kp.linear = 1;
@@ -1076,24 +1077,27 @@ class Engine : public EngineBase {
     }
 
     // solve_pressure of the hydrostatic set (pressure.cpp:142-170, 229-298)
-    void hyd_solve(double step)
+    // (edges: with the lateral copies of the forecast winds, unless the
+    // advection launch has made them)
+    void hyd_solve(double step, bool edges = true)
     {
         KFields<T> F = fields();
-        ProfScope ps(this, PC_THOMAS, 8);
-        const long e3 = 2L * (NX + NY - 2) * (NZ - 2);
-        k_mirror_edges<T><<<cdiv(e3, 256), 256, 0, stream>>>(kp, F.P[FU], F.P[FV], F.P[FV]);
-        const long ncol = (long)(NX - 2) * (NY - 2);
+        ProfScope ps(this, PC_THOMAS, edges ? 6 : 5);
+        if (edges) {
+            const long e3 = 2L * (NX + NY - 2) * (NZ - 2);
+            k_mirror_edges<T><<<cdiv(e3, 256), 256, 0, stream>>>(kp, F.P[FU], F.P[FV], F.P[FV]);
+            launches++;
+        }
+        const int ncol = (NX - 2) * (NY - 2);
         const size_t hs = hyd_col_smem<T>(NZ);
         k_hyd_divavg<T><<<cdiv(ncol, HC), HC_THREADS, hs, stream>>>(kp, F, hyd, (T)step);
-        k_hyd_mirror2d<T><<<cdiv(2L * (NX + NY - 2), 256), 256, 0, stream>>>(kp, hyd.div);
         const size_t sm = 2 * (size_t)NX * hyd_L * sizeof(T2);
         const dim3 fb(hyd_L, std::max(1, 256 / hyd_L));
         k_hyd_fft<T><<<cdiv(NY, hyd_L), fb, sm, stream>>>(kp, hyd, plan_i, tw_i, 0, hyd_L);
-        k_hyd_thomas<T><<<cdiv(NX, 64), 64, 0, stream>>>(kp, hyd);
+        k_hyd_thomas<T><<<cdiv(NX, HT), HT_THREADS, hyd.tw ? 0 : hyd_thomas_smem<T>(NY), stream>>>(kp, hyd);
         k_hyd_fft<T><<<cdiv(NY, hyd_L), fb, sm, stream>>>(kp, hyd, plan_i, tw_i, 1, hyd_L);
         k_hyd_pi<T><<<cdiv(ncol, HC), HC_THREADS, hs, stream>>>(kp, F, hyd);
-        k_mirror_edges<T><<<cdiv(e3, 256), 256, 0, stream>>>(kp, pi, pi, pi);
-        launches += 8;
+        launches += 5;
     }
     void hyd_project(double step)
     {
@@ -1582,8 +1586,8 @@ class Engine : public EngineBase {
                 // Rutledge fall speeds read the solved Exner perturbation)
                 const bool ice = kp.ice;
                 const int scal = ADV_TH | (moist && !ice ? (ADV_Q | ADV_ZERO) : 0);
-                const bool side = overlap && !prof;
-                advect(st, ADV_UV | (side ? 0 : scal));
+                const bool side = overlap && !prof, fuse = use_march();
+                advect(st, ADV_UV | (side ? 0 : scal) | (fuse ? ADV_MIRROR : 0));
                 if (side) {  // with their column pass
                     fork();
                     OnSide os(this);
@@ -1593,7 +1597,7 @@ class Engine : public EngineBase {
                     if (moist && !ice) fs[FQV] = fs[FQC] = fs[FQR] = PF_ZERO | PF_SPONGE | PF_VBC;
                     post(fs, 9, st, true);
                 }
-                hyd_solve(st);
+                hyd_solve(st, !fuse);
                 hyd_project(st);
                 if (ice) {
                     const bool quad = adv_takes_ice();

@@ -31,7 +31,7 @@ struct HydArgs {
     // a warp of wavenumbers reads one row at a time)
     const T *pf, *rden;
     const T *ac;           // acoef [ny]
-    T *pw;                 // work of the back substitution, [2][ny+1][nx] (real and imaginary Q)
+    T *tw;                 // work of the tridiagonal solves where shared memory is too small, or null
     T *div;                // div_avg, [nx][ny]
     typename V2<T>::t *spec2;  // transformed div_avg, [ny][nx]
     T rhoavg;              // column-average density (column_average_density, initializer.cpp:1265-1282)
@@ -39,65 +39,64 @@ struct HydArgs {
 };
 
 // The column kernels below hold HC columns per block with their levels in
-// shared memory: the pointwise parts of each recurrence are formed by all
-// threads with loads coalesced along k, then one thread per column runs the
-// recurrence in the reference's order from shared memory.
-constexpr int HC = 16, HC_THREADS = 128;
+// shared memory, a warp per column at a time with lanes over the levels; the
+// pointwise parts of each recurrence (and its level factors) are formed by all
+// lanes, then one thread per column runs the bare recurrence in the
+// reference's order from shared memory.
+constexpr int HC = 16, HC_THREADS = 128, HC_WARPS = HC_THREADS / 32;
 
+// columns, and three rows of level factors
 template <typename T>
 __host__ __device__ constexpr size_t hyd_col_smem(int nz)
 {
-    return 2 * (size_t)HC * nz * sizeof(T);
+    return (2 * (size_t)HC + 3) * nz * sizeof(T);
+}
+
+// the columns that take column (i, j)'s value: itself and the lateral edges
+// that mirror it (mirror_boundaries, boundaries.cpp:331-379; a corner takes
+// the diagonal neighbour, as the reference's two passes leave it)
+template <typename F>
+__device__ __forceinline__ void with_mirrors(int nx, int ny, int i, int j, F f)
+{
+    const int ie = i == 1 ? 0 : i == nx - 2 ? nx - 1 : i, je = j == 1 ? 0 : j == ny - 2 ? ny - 1 : j;
+    f(i, j);
+    if (ie != i) f(ie, j);
+    if (je != j) f(i, je);
+    if (ie != i && je != j) f(ie, je);
 }
 
 // density-weighted column divergence of the forecast u, v (pressure.cpp:248-261)
+// with its lateral mirror copies
 template <typename T>
 __global__ void __launch_bounds__(HC_THREADS) k_hyd_divavg(KParams<T> p, KFields<T> F, HydArgs<T> h, T step)
 {
     extern __shared__ unsigned char hyd_smem[];
     T *term = (T *)hyd_smem;  // [HC][nz]
-    const int nyi = p.ny - 2, nz = p.nz;
-    const long ncol = (long)(p.nx - 2) * nyi, col0 = (long)blockIdx.x * HC;
+    const int nyi = p.ny - 2, nz = p.nz, lane = threadIdx.x & 31;
+    const int ncol = (p.nx - 2) * nyi, col0 = blockIdx.x * HC;
     const T *UP = F.P[FU], *VP = F.P[FV];
     const long sx = (long)p.ny * nz, sy = nz;
-    for (int w = threadIdx.x; w < HC * nz; w += blockDim.x) {
-        const int cl = w / nz, k = w % nz;
-        const long col = col0 + cl;
-        if (col >= ncol || k < 1 || k >= nz - 1) continue;
-        const int i = 1 + (int)(col / nyi), j = 1 + (int)(col % nyi);
-        const long c = gix(p.ny, nz, i, j, k);
-        term[cl * nz + k] =
-            p.rhou[k] * h.dzu[k] * ((UP[c + sx] - UP[c]) * p.one_d_dx + (VP[c + sy] - VP[c]) * p.one_d_dy);
+    for (int cl = threadIdx.x >> 5; cl < HC && col0 + cl < ncol; cl += HC_WARPS) {
+        const int col = col0 + cl, ci = col / nyi;
+        const long c0 = gix(p.ny, nz, 1 + ci, 1 + col - ci * nyi, 0);
+        for (int k = 1 + lane; k < nz - 1; k += 32) {
+            const long c = c0 + k;
+            term[cl * nz + k] =
+                p.rhou[k] * h.dzu[k] * ((UP[c + sx] - UP[c]) * p.one_d_dx + (VP[c + sy] - VP[c]) * p.one_d_dy);
+        }
     }
     __syncthreads();
-    const long col = col0 + threadIdx.x;
+    const int col = col0 + threadIdx.x;
     if (threadIdx.x >= HC || col >= ncol) return;
-    const int i = 1 + (int)(col / nyi), j = 1 + (int)(col % nyi);
     T d = T(0), zsum = T(0);
+#pragma unroll 8
     for (int k = 1; k < nz - 1; k++) {
         d += term[threadIdx.x * nz + k];
         zsum += h.dzu[k];
     }
     d /= (T(1004) * zsum * step * p.dt);
-    h.div[(long)i * p.ny + j] = d;
-}
-
-// mirror_boundaries_2d (boundaries.cpp:331-345): the edges take their
-// clamped interior neighbour (the corners the diagonal one, as the two
-// passes of the reference leave them)
-template <typename T>
-__global__ void k_hyd_mirror2d(KParams<T> p, T *s)
-{
-    const int ne = 2 * (p.nx + p.ny - 2);
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= ne) return;
-    int i, j, e = t;
-    if (e < p.ny) { i = 0; j = e; }
-    else if ((e -= p.ny) < p.ny) { i = p.nx - 1; j = e; }
-    else if ((e -= p.ny) < p.nx - 2) { i = 1 + e; j = 0; }
-    else { e -= p.nx - 2; i = 1 + e; j = p.ny - 1; }
-    const int si = min(max(i, 1), p.nx - 2), sj = min(max(j, 1), p.ny - 2);
-    s[(long)i * p.ny + j] = s[(long)si * p.ny + sj];
+    const int ci = col / nyi;
+    with_mirrors(p.nx, p.ny, 1 + ci, 1 + col - ci * nyi, [&](int i, int j) { h.div[(long)i * p.ny + j] = d; });
 }
 
 // transform along x of L y-lines (block (L, any)): forward from div_avg with
@@ -144,73 +143,103 @@ __global__ void k_hyd_fft(KParams<T> p, HydArgs<T> h, FftPlan P, const typename 
         }
 }
 
-// the tridiagonal solve along y of one x-wavenumber (pressure.cpp:675-700),
-// real and imaginary parts, with the precomputed factors: each step
-// of the recurrence is a multiply-subtract and a multiply by 1/denom (the
-// reference divides by denom; the two differ by an ulp, well inside the
-// transform's own rounding)
+// the tridiagonal solves along y of HT x-wavenumbers (pressure.cpp:675-700),
+// real and imaginary parts, with the precomputed factors: each step of the
+// recurrence is a multiply-subtract and a multiply by 1/denom (the reference
+// divides by denom; the two differ by an ulp, well inside the transform's own
+// rounding).  Rows are [j][i]: the block stages its wavenumbers' rows and
+// factors into shared memory at once, then two threads a wavenumber (real and
+// imaginary) run the bare chain of 2 NY steps from there.  With a thread per
+// wavenumber reading its rows from L2 in chunks it took 22 us at 128x128 in
+// FP32; now 8.
+constexpr int HT = 4, HT_THREADS = 128;
 template <typename T>
-__global__ void k_hyd_thomas(KParams<T> p, HydArgs<T> h)
+__host__ __device__ constexpr size_t hyd_thomas_smem(int ny)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= p.nx) return;
+    return (size_t)HT * ny * 4 * sizeof(T);
+}
+// v: [j][HT] (re, im), the rows, then Q, then the solution
+template <typename T>
+__device__ __forceinline__ void hyd_thomas_body(const KParams<T> &p, const HydArgs<T> &h, T *v)
+{
     typedef typename V2<T>::t T2;
-    const int nj = p.ny, nx = p.nx;
-    // rows are [j][i]: each step of the recurrence is one coalesced row for
-    // the warp; distinct arrays, so the loads of later rows may be issued
-    // before the stores of earlier ones
-    T *__restrict__ Qr = h.pw + i;
-    T *__restrict__ Qi = h.pw + (long)(nj + 1) * nx + i;
-    const T *__restrict__ P = h.pf + i;
-    const T *__restrict__ R = h.rden + i;
-    const T *__restrict__ ac = h.ac;
-    T2 *__restrict__ x = h.spec2 + i;
-    // each chunk's rows are loaded before its steps run, so a chunk waits on
-    // memory once rather than once per step
-    constexpr int CH = 16;
-    T qr = T(0), qi = T(0);
-    for (int j0 = 0; j0 < nj; j0 += CH) {
-        T2 v[CH];
-        T r[CH], av[CH];
+    const int nj = p.ny, nx = p.nx, i0 = blockIdx.x * HT, nt = min(HT, nx - i0);
+    T *r = v + (size_t)2 * HT * nj;             // [j][HT]: 1/denom
+    T *pf = r + (size_t)HT * nj;                // [j][HT]: P[j+1]
+    for (int w = threadIdx.x; w < HT * nj; w += HT_THREADS) {
+        const int j = w / HT, t = min(w % HT, nt - 1);
+        const long g = (long)j * nx + i0 + t;
+        const T2 x = h.spec2[g];
+        v[2 * w] = x.x;
+        v[2 * w + 1] = x.y;
+        r[w] = h.rden[g];
+        pf[w] = h.pf[g + nx];
+    }
+    __syncthreads();
+    if (threadIdx.x < 2 * HT) {
+        // chunks of rows are read before their steps run, so a chunk waits on
+        // shared memory once
+        constexpr int CH = 8;
+        const int t = threadIdx.x >> 1;
+        T *c = v + threadIdx.x;
+        const T last = c[2 * HT * (nj - 1)];  // the last row keeps its transformed value
+        const T a1 = h.ac[1];                 // acoef: 0 in row 0, 1/dy^2 above
+        T q = T(0);
+        for (int j0 = 0; j0 < nj; j0 += CH) {
+            T x[CH], rj[CH];
 #pragma unroll
-        for (int t = 0; t < CH; t++) {
-            const int j = min(j0 + t, nj - 1);
-            v[t] = x[(long)j * nx];
-            r[t] = R[(long)j * nx];
-            av[t] = ac[j];
+            for (int e = 0; e < CH; e++) {
+                const int j = min(j0 + e, nj - 1);
+                x[e] = c[2 * HT * j];
+                rj[e] = r[HT * j + t];
+            }
+#pragma unroll
+            for (int e = 0; e < CH; e++) {
+                const int j = j0 + e;
+                if (j < nj) {
+                    q = (x[e] - (j == 0 ? T(0) : a1) * q) * rj[e];
+                    c[2 * HT * j] = q;
+                }
+            }
         }
+        c[2 * HT * (nj - 1)] = last;
+        T s = last;
+        for (int j0 = nj - 2; j0 >= 0; j0 -= CH) {
+            T x[CH], f[CH];
 #pragma unroll
-        for (int t = 0; t < CH; t++) {
-            const int j = j0 + t;
-            if (j < nj) {
-                qr = (v[t].x - av[t] * qr) * r[t];
-                qi = (v[t].y - av[t] * qi) * r[t];
-                Qr[(long)(j + 1) * nx] = qr;
-                Qi[(long)(j + 1) * nx] = qi;
+            for (int e = 0; e < CH; e++) {
+                const int j = max(j0 - e, 0);
+                x[e] = c[2 * HT * j];
+                f[e] = pf[HT * j + t];
+            }
+#pragma unroll
+            for (int e = 0; e < CH; e++) {
+                const int j = j0 - e;
+                if (j >= 0) {
+                    s = f[e] * s + x[e];
+                    c[2 * HT * j] = s;
+                }
             }
         }
     }
-    T xr = x[(long)(nj - 1) * nx].x, xi = x[(long)(nj - 1) * nx].y;
-    for (int j1 = nj - 2; j1 >= 0; j1 -= CH) {
-        T pj[CH], qrj[CH], qij[CH];
-#pragma unroll
-        for (int t = 0; t < CH; t++) {
-            const int j = max(j1 - t, 0);
-            pj[t] = P[(long)(j + 1) * nx];
-            qrj[t] = Qr[(long)(j + 1) * nx];
-            qij[t] = Qi[(long)(j + 1) * nx];
-        }
-#pragma unroll
-        for (int t = 0; t < CH; t++) {
-            const int j = j1 - t;
-            if (j >= 0) {
-                xr = pj[t] * xr + qrj[t];
-                xi = pj[t] * xi + qij[t];
-                x[(long)j * nx].x = xr;
-                x[(long)j * nx].y = xi;
-            }
-        }
+    __syncthreads();
+    for (int w = threadIdx.x; w < HT * nj; w += HT_THREADS) {
+        const int j = w / HT, t = w % HT;
+        if (t >= nt) continue;
+        T2 o;
+        o.x = v[2 * w];
+        o.y = v[2 * w + 1];
+        h.spec2[(long)j * nx + i0 + t] = o;
     }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(HT_THREADS) k_hyd_thomas(KParams<T> p, HydArgs<T> h)
+{
+    extern __shared__ unsigned char hyd_smem[];
+    // (lines too long for shared memory use a device buffer)
+    if (h.tw) hyd_thomas_body(p, h, h.tw + (size_t)blockIdx.x * 4 * HT * p.ny);
+    else hyd_thomas_body(p, h, (T *)hyd_smem);
 }
 
 // hydrostatic_pressure (pressure.cpp:453-537) from the current theta (and
@@ -220,52 +249,76 @@ template <typename T>
 __global__ void __launch_bounds__(HC_THREADS) k_hyd_pi(KParams<T> p, KFields<T> F, HydArgs<T> h)
 {
     extern __shared__ unsigned char hyd_smem[];
-    const int nyi = p.ny - 2, nz = p.nz;
-    T *g = (T *)hyd_smem;   // [HC][nz]: theta (times the water loading) / tbv^2
-    T *ps = g + HC * nz;    // [HC][nz]: the integral, then the total
-    const long ncol = (long)(p.nx - 2) * nyi, col0 = (long)blockIdx.x * HC;
+    const int nyi = p.ny - 2, nz = p.nz, lane = threadIdx.x & 31;
+    T *g = (T *)hyd_smem;   // [HC][nz]: theta (times the water loading) / tbv^2, then the integral
+    T *ps = g + HC * nz;    // [HC][nz]: the integral's steps
+    T *wt = ps + HC * nz;   // [nz]: rhou tbv
+    T *dzu = wt + nz;       // [nz]
+    T *dzw = dzu + nz;      // [nz]
+    const int ncol = (p.nx - 2) * nyi, col0 = blockIdx.x * HC;
     const T *TH = F.cur[FTH], *QV = F.cur[FQV], *QC = F.cur[FQC], *QR = F.cur[FQR];
     T *PI = F.pi;
-    for (int w = threadIdx.x; w < HC * nz; w += blockDim.x) {
-        const int cl = w / nz, k = w % nz;
-        const long col = col0 + cl;
-        if (col >= ncol || k < 1 || k >= nz - 1) continue;
-        const long c = gix(p.ny, nz, 1 + (int)(col / nyi), 1 + (int)(col % nyi), k);
-        T fac = p.moist ? (T(1.) + T(0.61) * QV[c] - QC[c] - QR[c]) : T(1);
-        if (p.ice) fac = fac - F.cur[FQS][c] - F.cur[FQI][c];  // pressure.cpp:459-475
-        g[cl * nz + k] = (TH[c] * fac) / (p.tbv[k] * p.tbv[k]);
+    const T gcp = T(9.8 / 1004.0);
+    for (int k = threadIdx.x; k < nz; k += HC_THREADS) {
+        wt[k] = p.rhou[k] * p.tbv[k];
+        dzu[k] = h.dzu[k];
+        dzw[k] = h.dzw[k];
+    }
+    for (int cl = threadIdx.x >> 5; cl < HC && col0 + cl < ncol; cl += HC_WARPS) {
+        const int col = col0 + cl, ci = col / nyi;
+        const long c0 = gix(p.ny, nz, 1 + ci, 1 + col - ci * nyi, 0);
+        T *gc = g + cl * nz, *pc = ps + cl * nz;
+        for (int k = 1 + lane; k < nz - 1; k += 32) {
+            const long c = c0 + k;
+            T fac = p.moist ? (T(1.) + T(0.61) * QV[c] - QC[c] - QR[c]) : T(1);
+            if (p.ice) fac = fac - F.cur[FQS][c] - F.cur[FQI][c];  // pressure.cpp:459-475
+            gc[k] = (TH[c] * fac) / (p.tbv[k] * p.tbv[k]);
+        }
+        __syncwarp();
+        // the steps of the downward integral, without the layer's depth
+        for (int k = 1 + lane; k < nz - 1; k += 32)
+            pc[k] = k == nz - 2 ? T(0.5) * gcp * gc[k] : T(0.5) * gcp * (gc[k + 1] + gc[k]);
     }
     __syncthreads();
-    const T gcp = T(9.8 / 1004.0);
-    const int cl = threadIdx.x;
-    const long col = col0 + cl;
+    const int cl = threadIdx.x, col = col0 + cl;
     if (cl < HC && col < ncol) {
-        const int i = 1 + (int)(col / nyi), j = 1 + (int)(col % nyi);
-        const T *gc = g + cl * nz;
-        T *pc = ps + cl * nz;
-        T up = -T(0.5) * gcp * gc[nz - 2] * h.dzw[nz - 1];
+        const int ci = col / nyi, i = 1 + ci, j = 1 + col - ci * nyi;
+        const T *__restrict__ st = ps + cl * nz;  // the steps; the integral replaces the loads in g
+        T *__restrict__ pc = g + cl * nz;
+        T up = -st[nz - 2] * dzw[nz - 1];
         pc[nz - 2] = up;
+#pragma unroll 8
         for (int k = nz - 3; k > 0; k--) {
-            up = up - T(0.5) * gcp * (gc[k + 1] + gc[k]) * h.dzw[k + 1];
+            up = fma_(-st[k], dzw[k + 1], up);
             pc[k] = up;
         }
         T avg = T(0), zsum = T(0);
+#pragma unroll 8
         for (int k = 1; k < nz - 1; k++) {
-            avg += p.rhou[k] * p.tbv[k] * pc[k] * h.dzu[k];
-            zsum += h.dzu[k];
+            avg = fma_(mul_(wt[k], pc[k]), dzu[k], avg);
+            zsum += dzu[k];
         }
         avg /= zsum;
         pc[0] = avg;
         pc[nz - 1] = (h.div[(long)i * p.ny + j] - avg) / h.rhoavg;
     }
     __syncthreads();
-    for (int w = threadIdx.x; w < HC * nz; w += blockDim.x) {
-        const int c2 = w / nz, k = w % nz;
-        const long cc = col0 + c2;
-        if (cc >= ncol) continue;
-        const long c = gix(p.ny, nz, 1 + (int)(cc / nyi), 1 + (int)(cc % nyi), k);
-        const T *pc = ps + c2 * nz;
-        PI[c] = (k == 0 || k == nz - 1) ? pc[k] : pc[k] + pc[nz - 1];
+    for (int c2 = threadIdx.x >> 5; c2 < HC && col0 + c2 < ncol; c2 += HC_WARPS) {
+        const int cc = col0 + c2, ci = cc / nyi;
+        const T *pc = g + c2 * nz;
+        const T lid = pc[nz - 1];
+        // levels 1..NZ-2 to the edges that mirror the column as well
+        with_mirrors(p.nx, p.ny, 1 + ci, 1 + cc - ci * nyi, [&](int i, int j) {
+            const bool edge = i == 0 || j == 0 || i == p.nx - 1 || j == p.ny - 1;
+            T *o = PI + gix(p.ny, nz, i, j, 0);
+            for (int k = lane; k < nz; k += 32) {
+                if (k == 0 || k == nz - 1) {
+                    if (!edge) o[k] = pc[k];
+                } else {
+                    o[k] = pc[k] + lid;
+                }
+            }
+        });
     }
 }
 
@@ -291,40 +344,49 @@ template <typename T>
 __global__ void __launch_bounds__(HC_THREADS) k_hyd_w(KParams<T> p, KFields<T> F, HydArgs<T> h)
 {
     extern __shared__ unsigned char hyd_smem[];
-    const int nyi = p.ny - 2, nz = p.nz;
-    T *dv = (T *)hyd_smem;  // [HC][nz]: the horizontal convergence of level k
-    T *ws = dv + HC * nz;   // [HC][nz]: w
-    const long ncol = (long)(p.nx - 2) * nyi, col0 = (long)blockIdx.x * HC;
+    const int nyi = p.ny - 2, nz = p.nz, lane = threadIdx.x & 31;
+    T *dv = (T *)hyd_smem;   // [HC][nz]: the convergence term of level k (the level above its cell)
+    T *ws = dv + HC * nz;    // [HC][nz]: w
+    T *ra = ws + HC * nz;    // [nz]: rhow[k-1]/rhow[k]
+    T *rb = ra + nz;         // [nz]: rhou[k-1]/rhow[k]
+    const int ncol = (p.nx - 2) * nyi, col0 = blockIdx.x * HC;
     const T *UP = F.P[FU], *VP = F.P[FV];
     const long sx = (long)p.ny * nz, sy = nz;
-    for (int w = threadIdx.x; w < HC * nz; w += blockDim.x) {
-        const int cl = w / nz, k = w % nz;
-        const long col = col0 + cl;
-        if (col >= ncol || k < 1 || k >= nz - 2) continue;
-        const long c = gix(p.ny, nz, 1 + (int)(col / nyi), 1 + (int)(col % nyi), k);
-        dv[cl * nz + k] = -(UP[c + sx] - UP[c]) * p.one_d_dx - (VP[c + sy] - VP[c]) * p.one_d_dy;
+    for (int k = 2 + threadIdx.x; k < nz - 1; k += HC_THREADS) {
+        ra[k] = p.rhow[k - 1] / p.rhow[k];
+        rb[k] = p.rhou[k - 1] / p.rhow[k];
+    }
+    __syncthreads();
+    for (int cl = threadIdx.x >> 5; cl < HC && col0 + cl < ncol; cl += HC_WARPS) {
+        const int col = col0 + cl, ci = col / nyi;
+        const long c0 = gix(p.ny, nz, 1 + ci, 1 + col - ci * nyi, 0);
+        for (int k = 2 + lane; k < nz - 1; k += 32) {
+            const long c = c0 + k - 1;
+            const T d = -(UP[c + sx] - UP[c]) * p.one_d_dx - (VP[c + sy] - VP[c]) * p.one_d_dy;
+            dv[cl * nz + k] = rb[k] * d * h.dz / p.mu[k - 1];
+        }
     }
     __syncthreads();
     const int cl = threadIdx.x;
     if (cl < HC && col0 + cl < ncol) {
-        T *wc = ws + cl * nz;
-        const T *dc = dv + cl * nz;
+        T *__restrict__ wc = ws + cl * nz;
+        const T *__restrict__ dc = dv + cl * nz;
         wc[0] = T(0);
         wc[1] = T(0);
         wc[nz - 1] = T(0);
         T w = T(0);
+#pragma unroll 8
         for (int k = 2; k < nz - 1; k++) {
-            w = (p.rhow[k - 1] / p.rhow[k]) * w + (p.rhou[k - 1] / p.rhow[k]) * dc[k - 1] * h.dz / p.mu[k - 1];
+            w = fma_(ra[k], w, dc[k]);
             wc[k] = w;
         }
     }
     __syncthreads();
     T *W = F.cur[FW];
-    for (int w = threadIdx.x; w < HC * nz; w += blockDim.x) {
-        const int c2 = w / nz, k = w % nz;
-        const long cc = col0 + c2;
-        if (cc >= ncol) continue;
-        W[gix(p.ny, nz, 1 + (int)(cc / nyi), 1 + (int)(cc % nyi), k)] = ws[c2 * nz + k];
+    for (int c2 = threadIdx.x >> 5; c2 < HC && col0 + c2 < ncol; c2 += HC_WARPS) {
+        const int cc = col0 + c2, ci = cc / nyi;
+        T *o = W + gix(p.ny, nz, 1 + ci, 1 + cc - ci * nyi, 0);
+        for (int k = lane; k < nz; k += 32) o[k] = ws[c2 * nz + k];
     }
 }
 

@@ -586,7 +586,7 @@ __global__ void __launch_bounds__(AM_THREADS, MB)
         const long ntot = 2L * (p.nx + p.ny - 2) * (p.nz - 2);
         const long b = ((long)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
         for (long t = b * AM_THREADS + threadIdx.x; t < ntot; t += nt)
-            mirror_edges_body(p, F.P[FU], F.P[FV], F.P[FW], t);
+            mirror_edges_body(p, F.P[FU], F.P[FV], p.hydrostatic ? F.P[FV] : F.P[FW], t);
     }
     const int jb = by_job ? blockIdx.z : blockIdx.x, jt = by_job ? blockIdx.x : blockIdx.z;
     march_body(p, F, g, (int)((jobs >> (4 * jb)) & 15ull), blockIdx.y, jt, step, sdtg, what);
