@@ -1062,12 +1062,11 @@ class Engine : public EngineBase {
         const int order = cfg.diffusion_order;
         if (!diff_tend || !diff_w || (order != 2 && order != 4 && order != 6)) return;
         ProfScope ps(this, PC_DIFFUSION, 1);
-        const long tot = N * nprog;
-        const int nb = (int)std::min((tot + 255) / 256, 152L * 16);
+        const int nb = (int)std::min((N + 255) / 256, 152L * 16);
         KFields<T> F = fields();
         DiffOut<T> o;
         for (int f = 0; f < 9; f++) o.out[f] = (f < nprog && !(f == FW && hyd.div)) ? diff_buf[f] : nullptr;
-        k_diffuse_into<T><<<nb, 256, 0, stream>>>(kp, F, o, nprog, order, (T)cfg.kdiffh, (T)cfg.kdiffv, diff_w,
+        k_diffuse_into<T><<<dim3(nb, nprog), 256, 0, stream>>>(kp, F, o, nprog, order, (T)cfg.kdiffh, (T)cfg.kdiffv, diff_w,
                                                   (T)step);
         // the diffused copy becomes the start-of-step slot; two steps swap
         // back, so a captured two-step graph leaves the pointers as it found them

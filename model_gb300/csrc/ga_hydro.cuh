@@ -328,11 +328,9 @@ template <typename T>
 __global__ void __launch_bounds__(256) k_hyd_project(KParams<T> p, KFields<T> F, T step)
 {
     const int nzi = p.nz - 2, nyi = p.ny - 2;
-    const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long)(p.nx - 2) * nyi * nzi) return;
-    const int k = 1 + (int)(t % nzi);
-    const int j = 1 + (int)((t / nzi) % nyi);
-    const int i = 1 + (int)(t / ((long)nzi * nyi));
+    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;  // fewer than 2^31 points
+    if (t >= (unsigned)((p.nx - 2) * nyi * nzi)) return;
+    const int col = (int)t / nzi, k = 1 + (int)t - col * nzi, i = 1 + col / nyi, j = 1 + col % nyi;
     const long c = gix(p.ny, p.nz, i, j, k), sx = (long)p.ny * p.nz, sy = p.nz;
     const T *PI = F.pi;
     F.P[FU][c] = F.P[FU][c] - step * (p.dtx * T(1004) * p.tbv[k] * (PI[c] - PI[c - sx]));

@@ -2885,15 +2885,13 @@ template <typename T>
 __global__ void __launch_bounds__(256) k_diffuse_into(KParams<T> p, KFields<T> F, DiffOut<T> o, int nf, int order,
                                                       T kh, T kv, const T *dw, T step)
 {
-    const long per = p.n, tot = per * nf;
-    const long sx = (long)p.ny * p.nz, sy = p.nz;
-    for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < tot; t += (long)gridDim.x * blockDim.x) {
-        const int f = (int)(t / per);
-        const long c = t - f * per;
-        T *out = o.out[f];
-        if (!out) continue;  // a field left alone (w of the hydrostatic set)
-        const T *v = F.M[f];
-        const int k = (int)(c % p.nz), j = (int)((c / p.nz) % p.ny), i = (int)(c / sx);
+    // a field per grid row: fewer than 2^31 points each, 32-bit indices
+    const int f = blockIdx.y, n = (int)p.n, sx = p.ny * p.nz, sy = p.nz;
+    T *out = o.out[f];
+    if (!out) return;  // a field left alone (w of the hydrostatic set)
+    const T *v = F.M[f];
+    for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < (unsigned)n; t += gridDim.x * blockDim.x) {
+        const int c = (int)t, col = c / p.nz, k = c - col * p.nz, i = col / p.ny, j = col - i * p.ny;
         if (i < 3 || i >= p.nx - 3 || j < 3 || j >= p.ny - 3 || k < 1 || k >= p.nz - 1) {
             out[c] = v[c];
             continue;
