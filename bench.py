@@ -49,9 +49,9 @@ L2_FLUSH_BYTES = 256 << 20
 # Advection with a basic state of height only (every bench workload): the
 # current and start-of-step fields in, the forecast (and the fall speed) out;
 # the basic state is a per-level table.
-PASSES_DRY = {"advect": 12, "div_fft_y": 5, "fft_x": 4, "thomas": 4, "ifft_y_pi": 3, "post": 9,
+PASSES_DRY = {"advect": 12, "div_fft_y": 4, "fft_x": 2, "thomas": 2, "ifft_y_pi": 2, "post": 9,
               "kessler": 0}
-PASSES_MOIST = {"advect": 22, "div_fft_y": 5, "fft_x": 4, "thomas": 4, "ifft_y_pi": 3, "post": 16,
+PASSES_MOIST = {"advect": 22, "div_fft_y": 4, "fft_x": 2, "thomas": 2, "ifft_y_pi": 2, "post": 16,
                 "kessler": 12}
 # DRAM bytes per launch (read + write) of the dominant kernel, copied from one
 # ncu capture of the bench command (cold cache) into this table; a run does not
