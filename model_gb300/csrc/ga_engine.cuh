@@ -1163,7 +1163,8 @@ class Engine : public EngineBase {
             // against 3.5) where two blocks of it fit an SM (192x128x32, dry:
             // 0.457 against 0.477 ms); with six fields' faces only one does
             const bool wide = sizeof(T) == 8 && adv_ti == ADV_TI && adv_tj == ADV_TJ && !adv_tuned &&
-                              advect_tile_smem(4, 8, NZ, sizeof(T), what) <= 110 * 1024;
+                              advect_tile_smem(4, 8, NZ, sizeof(T), what) <= 110 * 1024 &&
+                              cdiv(NX - 6, 4) * cdiv(NY - 6, 8) >= 4 * nsm;  // (a small grid needs the blocks)
             if (wide) launch_advect_tile<4, 8>(st, sg, what);
             else if (adv_ti == 2) launch_advect_tile<2, 4>(st, sg, what);
             else if (adv_tj == 2) launch_advect_tile<4, 2>(st, sg, what);
