@@ -1212,8 +1212,8 @@ class Engine : public EngineBase {
             if constexpr (sizeof(T) == 4) pair = sx_pair && pair_ok();
             if (pair) {
                 if constexpr (sizeof(T) == 4) {
-                    const int bh = std::min((nl + 1) / 2, 32);
-                    k_spectral_x_pair<T><<<2 * kp.nh, dim3(bh, std::max(1, sx_threads / bh)), smem_sxp, stream>>>(
+                    const int bh = std::min((nl + 1) / 2, 32), nt = std::min(sx_threads, SX_PAIR_THREADS);
+                    k_spectral_x_pair<T><<<2 * kp.nh, dim3(bh, std::max(1, nt / bh)), smem_sxp, stream>>>(
                         kp, spec, plan_i, tw_i, sx_pair_layout(NZ));
                 }
             } else if (sx_threads > 512) {

@@ -1146,9 +1146,13 @@ __host__ inline size_t sx_pair_smem(int ni, int nz)
     return (2 * (size_t)ni * L.ps + (size_t)((ni + 1) / 2) * L.xs) * sizeof(float2);
 }
 
+// threads of a block at most: the default block of the single kernel (up to
+// 1024 threads) is more than this kernel's 72 registers a thread allow (896),
+// and the autotuner offers it 256 and 512
+constexpr int SX_PAIR_THREADS = 512;
 template <typename T>
-__global__ void __cluster_dims__(2, 1, 1) k_spectral_x_pair(KParams<T> p, typename V2<T>::t *spec, FftPlan pi,
-                                                           const typename V2<T>::t *tw, SxPair lay)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(SX_PAIR_THREADS)
+    k_spectral_x_pair(KParams<T> p, typename V2<T>::t *spec, FftPlan pi, const typename V2<T>::t *tw, SxPair lay)
 {
     static_assert(sizeof(T) == 4, "the paired x kernel is FP32");
     namespace cg = cooperative_groups;
