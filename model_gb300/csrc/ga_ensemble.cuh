@@ -683,7 +683,8 @@ class Ensemble : public EnsembleBase {
             launch_sx();
             kb_ifft_y_pi<T><<<grid[EK_IFFTY], dim3(8, 32), smem[EK_IFFTY], stream>>>(d_p, F, d_aux, d_pre[EK_IFFTY],
                                                                                      nmem);
-            const int fu = PF_PROJECT | PF_SPONGE | PF_VBC, ft = PF_SPONGE | PF_VBC, fq = PF_ZERO | PF_SPONGE | PF_VBC;
+            const int fu = PF_PROJECT | PF_SPONGE | PF_VBC, ft = PF_SPONGE | PF_VBC;
+            const int fq = moist ? PF_ZERO | PF_SPONGE | PF_VBC : 0;  // (dry members have no moisture buffers)
             launch_post(F, make_int4(fu, fu, fu, ft), make_int4(fq, fq, fq, 0), st);
             launches += 5 + sx_launches();
             if (s < 2) swap_all();
@@ -693,7 +694,8 @@ class Ensemble : public EnsembleBase {
             kb_kessler<T><<<grid[EK_KES], 128, 0, stream>>>(d_p, F, d_pre[EK_KES], nmem, d_err);
             launches++;
         }
-        const int fu = PF_SPONGE | PF_VBC | PF_RAYLEIGH | PF_WRITE_M, fq = PF_SPONGE | PF_VBC | PF_WRITE_M;
+        const int fu = PF_SPONGE | PF_VBC | PF_RAYLEIGH | PF_WRITE_M;
+        const int fq = moist ? PF_SPONGE | PF_VBC | PF_WRITE_M : 0;
         launch_post(F, make_int4(fu, fu, fu, fu), make_int4(fq, fq, fq, 0), 1.0);
         launches++;
         swap_all();
