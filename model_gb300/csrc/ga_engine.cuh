@@ -72,6 +72,7 @@ class Engine : public EngineBase {
     T *btab = nullptr, *mtab = nullptr;
     T *bface = nullptr;  // both upwind values of the basic-state faces (FP64)
     bool bface_tried = false;
+    bool bar_out = false;  // the caller holds a device pointer to a field behind them and may write there between steps
     long long graph_launches[2] = {0, 0};
     bool use_graphs = true;
     int status = GA_OK;
@@ -705,6 +706,10 @@ class Engine : public EngineBase {
     {
         if (field == GA_ACCRAIN) return accrain;
         if (field == GA_ACCSNOW) return accsnow;
+        if (field == GA_UBAR || field == GA_VBAR || field == GA_THBAR || field == GA_QBAR) {
+            bar_out = true;
+            drop_faces();
+        }
         long n;
         return host_field(field, slot, &n);
     }
@@ -837,6 +842,18 @@ class Engine : public EngineBase {
         if (lin) lin->drop_graphs();
     }
 
+    // gives the stored basic-state faces back; from then on they are evaluated
+    void drop_faces()
+    {
+        if (!bface) return;
+        cudaSetDevice(device);
+        cudaStreamSynchronize(stream);
+        drop_graphs();
+        cudaFree(bface);
+        bface = nullptr;
+        kp.bface = nullptr;
+    }
+
     // per-level basic-state tables (k_base_tables) when the basic state is
     // horizontally uniform; rebuilt after any basic-state field changes
     void refresh_base()
@@ -860,7 +877,9 @@ class Engine : public EngineBase {
         }
         kp.bface = nullptr;
         if constexpr (sizeof(T) == 8) {
-            if (!adv && !cfg.linear_model) {  // (without the memory for it the faces are evaluated each time)
+            // (without the memory for it, or where the caller may change the
+            // basic state unseen, the faces are evaluated each time)
+            if (!adv && !cfg.linear_model && !bar_out) {
                 const int nfb = kp.moist ? 4 : 3, src[4] = {0, 1, 3, 4};
                 if (!bface && !bface_tried && cudaMalloc(&bface, (size_t)nfb * 6 * N * sizeof(T)) != cudaSuccess) {
                     bface = nullptr;
