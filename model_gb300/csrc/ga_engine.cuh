@@ -1052,6 +1052,17 @@ class Engine : public EngineBase {
     // the marching kernel applies: FP32, basic state a function of height,
     // whole quads of levels
     bool use_march() const { return sizeof(T) == 4 && adv_march && kp.ubase_adv && NZ % 4 == 0; }
+    // A launch that keeps the clipping record takes a tile's three moisture
+    // fields one after another in the marching kernel: a chain that small flat
+    // grids wait for, so those use the four-level tile kernel.  Moist adjoint
+    // of four steps, tile against marching kernel: 32x32x24 2.02 / 2.21 ms,
+    // 64x64x16 2.09 / 2.29, 64x64x32 2.33 / 2.50, 96x96x32 3.12 / 3.10;
+    // two tangent-linear steps: 64x64x32 0.94 / 0.98, 64x64x40 1.06 / 1.06,
+    // 32x32x64 1.05 / 0.99, 128x128x24 1.69 / 1.66.
+    bool record_by_quad() const
+    {
+        return adv_force == 0 && NZ <= 32 && N <= 300000 && adv_quad && quad_ok(adv_qi, adv_qj);
+    }
     // a four-level advection kernel runs that also takes the mirror copies,
     // and snow and ice in the moisture launch
     bool adv_takes_mirror() const { return use_march() || (adv_quad && quad_ok(adv_qi, adv_qj)); }
@@ -1164,7 +1175,7 @@ class Engine : public EngineBase {
     {
         const double sdtg = step * cfg.dt * 9.8 * 0.5;  // step*dt*grav*0.5, advection.cpp:330
         ProfScope ps(this, PC_ADVECT, 1);
-        if (use_march()) {
+        if (use_march() && !(qmask && (what & ADV_Q) && record_by_quad())) {
             launch_march((T)step, (T)sdtg, what);
         } else if (adv_quad && adv_tma && tma_ok(adv_tmc)) {
             launch_advect_tma_cand(adv_tmc, (T)step, (T)sdtg, what);
