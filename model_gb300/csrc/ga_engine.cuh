@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "ga_engine.h"
+#include "ga_tune.h"
 #include "ga_kernels.cuh"
 #include "ga_quad.cuh"
 #include "ga_march.cuh"
@@ -1999,19 +2000,26 @@ class Engine : public EngineBase {
                 sx_pair = bp;
             }
             // the unfused path (x FFT, Thomas, inverse x FFT) and its level
-            // tile, against the fused kernel where that fits
+            // tile: against the fused kernel where that fits, otherwise
+            // against the current tile, timed once more beside the others
             {
                 const int keep_psx = psx, keep_kt = KTx;
                 psx = 0;
-                int bkx = -1;
-                for (int kt = 1; kt <= 64 && kt <= 2 * (NZ - 2); kt <<= 1) {
-                    if (fft_bytes(kp.ni, kt, sizeof(T2)) > 200 * 1024) break;
-                    set_ktx(kt);
-                    const float t = timeit([&] { solve_pressure(1. / 3.); });
-                    if (t < bx || (keep_psx == 0 && bkx < 0)) { bx = std::min(bx, t); bkx = kt; }
-                }
-                set_ktx(bkx > 0 ? bkx : keep_kt);
-                if (bkx <= 0) psx = keep_psx;
+                auto solve = [&] {
+                    float t = 1e30f;
+                    for (int r = 0; r < 3; r++) t = std::min(t, timeit([&] { solve_pressure(1. / 3.); }));
+                    return t;
+                };
+                if (keep_psx == 0) bx = std::min(bx, solve());
+                const int kt = faster_tile(
+                    keep_psx == 0 ? keep_kt : 0, std::min(64, 2 * (NZ - 2)), bx,
+                    [&](int k) { return fft_bytes(kp.ni, k, sizeof(T2)) <= 200 * 1024; },
+                    [&](int k) {
+                        set_ktx(k);
+                        return solve();
+                    });
+                set_ktx(kt > 0 ? kt : keep_kt);
+                if (kt <= 0) psx = keep_psx;
                 if (psx == 0) std::snprintf(line, sizeof line, "x level tile %d, ", KTx);
                 else std::snprintf(line, sizeof line, "x fused%s, %d threads, ", sx_pair ? " (CTA pairs)" : "",
                                    sx_threads);

@@ -1,0 +1,27 @@
+// Choice of a level tile by its time (host).
+#pragma once
+
+namespace ga {
+
+// `keep`, whose time is `best`, unless another power of two up to kmax that
+// fits is faster by more than 0.5%, about what the least of three samples of one
+// tile varies by (a context already at its best tile must stay there).
+// keep 0: no tile yet, `best` is what a tile has to beat.  Returns the tile and
+// leaves its time in `best`.
+template <typename Fits, typename Time>
+inline int faster_tile(int keep, int kmax, float &best, Fits fits, Time time)
+{
+    const int stay = keep;
+    for (int kt = 1; kt <= kmax; kt <<= 1) {
+        if (!fits(kt)) break;
+        if (kt == stay) continue;
+        const float t = time(kt);
+        if (t < 0.995f * best) {
+            best = t;
+            keep = kt;
+        }
+    }
+    return keep;
+}
+
+}  // namespace ga
