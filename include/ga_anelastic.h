@@ -235,7 +235,11 @@ GA_API int ga_coriolis_build(int ny, double dy, double corner_lat, double *f_out
 /* Replaces initialize_serial's solver set-up: initialize_pressure_solver
  * (pressure.cpp:99), init_boundaries (boundaries.cpp:44), init_microphysics
  * (microphysics.cpp:41).  Allocates every device buffer (zeroed, as the
- * reference's calloc) and precomputes the spectral and sponge tables. */
+ * reference's calloc) and precomputes the spectral and sponge tables.  FP64
+ * contexts add tables that only save time, while half of the device's memory
+ * stays free: one field's worth for the vertical solves here and, on a basic
+ * state that varies horizontally, 18 (dry) or 24 (moist) fields' worth on the
+ * first step.  They are given back when an allocation of the context fails. */
 GA_API int ga_create(const ga_config *cfg, const ga_columns *cols, ga_ctx **out);
 GA_API int ga_destroy(ga_ctx *ctx);
 
@@ -309,7 +313,10 @@ GA_API long long ga_launch_count(ga_ctx *ctx);
 GA_API void *ga_stream(ga_ctx *ctx);
 
 /* Device pointer of a field buffer (FP64 or FP32 per the precision), for
- * callers that keep state resident on the GPU. */
+ * callers that keep state resident on the GPU.  A context whose pointer to a
+ * basic-state field is out keeps no faces of the basic state, so a horizontally
+ * varying one may be written between steps; tables of a basic state of height
+ * alone are formed again only by ga_set_field. */
 GA_API void *ga_field_device_ptr(ga_ctx *ctx, int field, int slot);
 
 /*

@@ -71,8 +71,16 @@ class Engine : public EngineBase {
     bool bar_uniform[6] = {false, false, false, false, false, false};
     bool btab_dirty = true;
     T *btab = nullptr, *mtab = nullptr;
-    T *bface = nullptr;  // both upwind values of the basic-state faces (FP64)
-    bool bface_tried = false;
+    // Device tables that make FP64 steps faster and that a context can do
+    // without: the elimination of the vertical systems (one field's worth; none
+    // in the hydrostatic set) and both upwind values of the basic-state faces
+    // (18 or 24 fields' worth, on a basic state that varies horizontally).
+    // Built while half of the device's memory stays free, given back when
+    // another allocation of the context needs the room; results are the same
+    // with and without.  GA_FP64_TABLES=0 keeps them out.
+    double *elim = nullptr;
+    T *bface = nullptr;
+    bool tables_on = true, bface_tried = false;
     bool bar_out = false;  // the caller holds a device pointer to a field behind them and may write there between steps
     long long graph_launches[2] = {0, 0};
     bool use_graphs = true;
@@ -244,7 +252,7 @@ class Engine : public EngineBase {
     X *dalloc(size_t n)
     {
         void *p = nullptr;
-        if (cudaMalloc(&p, n * sizeof(X) ? n * sizeof(X) : 1) != cudaSuccess) {
+        if (take(&p, n * sizeof(X) ? n * sizeof(X) : 1) != cudaSuccess) {
             status = GA_ERR_NOMEM;
             return nullptr;
         }
@@ -510,14 +518,16 @@ class Engine : public EngineBase {
             kp.mean_inv = upload(inv);
         }
 
+        if (const char *ev = std::getenv("GA_FP64_TABLES")) tables_on = std::strcmp(ev, "0") != 0;
         if (sizeof(T) == 8) {
             const int ncol = ni * nh;
-            double *zt = dalloc<double>((size_t)ncol * (NZ - 2)), *ft = dalloc<double>((size_t)ncol * (NZ - 2));
-            if (zt && ft) {
+            const size_t n = (size_t)ncol * (NZ - 2);
+            kp.th_eval = 1;
+            if (status == GA_OK && !c->hydrostatic && table((void **)&elim, 2 * n * sizeof(double))) {
                 k_thomas_table<<<cdiv(ncol, 128), 128>>>(ncol, NZ, kp.dx2, kp.hcoef, kp.rhou_d, kp.acoef_d, kp.ccoef_d,
-                                                         kp.vcoef_d, zt, ft);
-                kp.th_z = zt;
-                kp.th_f = ft;
+                                                         kp.vcoef_d, elim, elim + n);
+                kp.th_z = elim;
+                kp.th_f = elim + n;
             }
         }
 
@@ -635,6 +645,7 @@ class Engine : public EngineBase {
             if (g) cudaGraphExecDestroy(g);
         for (void *p : allocs) cudaFree(p);
         if (staging) cudaFree(staging);
+        if (elim) cudaFree(elim);
         if (bface) cudaFree(bface);
         if (h_err) cudaFreeHost(h_err);
         if (stream2) cudaStreamSynchronize(stream2);
@@ -717,7 +728,7 @@ class Engine : public EngineBase {
 
     int ensure_staging()
     {
-        if (!staging && cudaMalloc(&staging, N * sizeof(double)) != cudaSuccess) return GA_ERR_NOMEM;
+        if (!staging && take((void **)&staging, N * sizeof(double)) != cudaSuccess) return GA_ERR_NOMEM;
         return GA_OK;
     }
 
@@ -843,6 +854,23 @@ class Engine : public EngineBase {
         if (lin) lin->drop_graphs();
     }
 
+    // a table of the kind above: allocated where it leaves half of the memory free
+    bool table(void **p, size_t bytes)
+    {
+        size_t fr = 0, tot = 0;
+        *p = nullptr;
+        if (tables_on && cudaMemGetInfo(&fr, &tot) == cudaSuccess && fr >= bytes + tot / 2 &&
+            cudaMalloc(p, bytes) == cudaSuccess)
+            return true;
+        cudaGetLastError();
+        *p = nullptr;
+        return false;
+    }
+    size_t table_bytes() const
+    {
+        return (elim ? 2 * (size_t)kp.ni * kp.nh * (NZ - 2) * sizeof(double) : 0) +
+               (bface ? (size_t)(kp.moist ? 4 : 3) * 6 * N * sizeof(T) : 0);
+    }
     // gives the stored basic-state faces back; from then on they are evaluated
     void drop_faces()
     {
@@ -853,6 +881,30 @@ class Engine : public EngineBase {
         cudaFree(bface);
         bface = nullptr;
         kp.bface = nullptr;
+        btab_dirty = true;  // (an ensemble copies kp again)
+    }
+    void drop_tables()
+    {
+        drop_faces();
+        if (!elim) return;
+        cudaSetDevice(device);
+        cudaStreamSynchronize(stream);
+        drop_graphs();
+        cudaFree(elim);
+        elim = nullptr;
+        kp.th_z = kp.th_f = nullptr;
+        btab_dirty = true;
+    }
+    // cudaMalloc that gives the tables back where the device has no room left
+    cudaError_t take(void **p, size_t bytes)
+    {
+        cudaError_t e = cudaMalloc(p, bytes);
+        if (e != cudaSuccess && table_bytes()) {
+            cudaGetLastError();
+            drop_tables();
+            e = cudaMalloc(p, bytes);
+        }
+        return e;
     }
 
     // per-level basic-state tables (k_base_tables) when the basic state is
@@ -882,10 +934,7 @@ class Engine : public EngineBase {
             // basic state unseen, the faces are evaluated each time)
             if (!adv && !cfg.linear_model && !bar_out) {
                 const int nfb = kp.moist ? 4 : 3, src[4] = {0, 1, 3, 4};
-                if (!bface && !bface_tried && cudaMalloc(&bface, (size_t)nfb * 6 * N * sizeof(T)) != cudaSuccess) {
-                    bface = nullptr;
-                    cudaGetLastError();
-                }
+                if (!bface && !bface_tried) table((void **)&bface, (size_t)nfb * 6 * N * sizeof(T));
                 bface_tried = true;
                 if (bface) {
                     for (int b = 0; b < nfb; b++)
@@ -1833,7 +1882,8 @@ class Engine : public EngineBase {
         refresh_base();
         const int nsnap = nprog + 2;
         T *snap = nullptr;
-        if (cudaMalloc(&snap, (size_t)nsnap * N * sizeof(T)) != cudaSuccess) return GA_ERR_NOMEM;
+        if (take((void **)&snap, (size_t)nsnap * N * sizeof(T)) != cudaSuccess) return GA_ERR_NOMEM;
+        refresh_base();  // (with the faces given back)
         for (int f = 0; f < nprog; f++)
             cudaMemcpyAsync(snap + (size_t)f * N, buf[f][pi_[f]], N * sizeof(T), cudaMemcpyDeviceToDevice, stream);
         cudaMemcpyAsync(snap + (size_t)nprog * N, pi, N * sizeof(T), cudaMemcpyDeviceToDevice, stream);
@@ -2125,7 +2175,7 @@ class Engine : public EngineBase {
         cudaSetDevice(device);
         cudaMemsetAsync(d_err + 0, 0, 0, stream);
         int *flag = nullptr;
-        if (cudaMalloc(&flag, sizeof(int)) != cudaSuccess) return GA_ERR_NOMEM;
+        if (take((void **)&flag, sizeof(int)) != cudaSuccess) return GA_ERR_NOMEM;
         cudaMemsetAsync(flag, 0, sizeof(int), stream);
         for (int f = 0; f < nprog; f++)
             for (int s = 0; s < 3; s++) {

@@ -255,6 +255,12 @@ class Ensemble : public EnsembleBase {
         moist = cfgs[0].microphysics_option == 1;
         for (int m = 0; m < n; m++) {
             Engine<T> *e = new Engine<T>(&cfgs[m], &cols[m]);
+            if (e->status == GA_ERR_NOMEM && m > 0) {  // once more without the earlier members' tables
+                cudaGetLastError();
+                delete e;
+                for (auto *o : mem) o->drop_tables();
+                e = new Engine<T>(&cfgs[m], &cols[m]);
+            }
             if (e->status != GA_OK) {
                 *rc = e->status;
                 delete e;
@@ -464,7 +470,12 @@ class Ensemble : public EnsembleBase {
         size_t tot = 0;
         for (auto *e : mem) tot += (size_t)nf * e->N;
         T *snap = nullptr;
-        if (cudaMalloc(&snap, tot * sizeof(T)) != cudaSuccess) return GA_ERR_NOMEM;
+        if (cudaMalloc(&snap, tot * sizeof(T)) != cudaSuccess) {
+            cudaGetLastError();
+            for (auto *e : mem) e->drop_tables();
+            refresh_tables();
+            if (cudaMalloc(&snap, tot * sizeof(T)) != cudaSuccess) return GA_ERR_NOMEM;
+        }
         auto copy_all = [&](bool save) {
             size_t o = 0;
             for (auto *e : mem) {

@@ -46,8 +46,10 @@ struct KParams {
     const T *acoef, *ccoef, *vcoef;             // [nz]
     const double *acoef_d, *ccoef_d, *vcoef_d, *rhou_d;  // FP64 islands
     // FP64 contexts: the elimination of every wavenumber's system, [level][column]
-    // (columns p*nh + q, ncol = ni*nh): reciprocal pivots and upper factors, or null
+    // (columns p*nh + q, ncol = ni*nh): reciprocal pivots and upper factors, or
+    // null: evaluated in each solve (th_eval), with the same results
     const double *th_z, *th_f;
+    int th_eval;
     double dx2;
     T rhou1;
     int low_modes;  // |p|,|q| below this solve in FP64 (FP32 contexts)
@@ -1632,20 +1634,27 @@ __device__ void thomas_column(const KParams<T> &p, typename V2<T>::t *x, A *Fw, 
 // reciprocal pivots z and upper factors F do not change during a run.  A solve
 // then multiplies where it divided (FP64 divisions are chains of dependent
 // operations on a pipe of two lanes an SM).
-static __global__ void k_thomas_table(int ncol, int nz, double dx2, const double *hcoef, const double *rhou,
-                                      const double *ac, const double *cc, const double *vc, double *zt, double *ft)
+template <typename Put>
+__device__ __forceinline__ void thomas_factors(int nz, double h, double dx2, const double *rhou, const double *ac,
+                                               const double *cc, const double *vc, Put put)
 {
-    const int col = blockIdx.x * blockDim.x + threadIdx.x;
-    if (col >= ncol) return;
-    const double h = hcoef[col];
     double Fk = 0.0;
     for (int k = 1; k < nz - 1; k++) {
         const double bk = rhou[k] * 2.0 * h / dx2 - vc[k];
         const double z = 1.0 / (k == 1 ? bk : bk - ac[k] * Fk);
         Fk = cc[k] * z;
-        zt[(long)(k - 1) * ncol + col] = z;
-        ft[(long)(k - 1) * ncol + col] = Fk;
+        put(k - 1, z, Fk);
     }
+}
+static __global__ void k_thomas_table(int ncol, int nz, double dx2, const double *hcoef, const double *rhou,
+                                      const double *ac, const double *cc, const double *vc, double *zt, double *ft)
+{
+    const int col = blockIdx.x * blockDim.x + threadIdx.x;
+    if (col >= ncol) return;
+    thomas_factors(nz, hcoef[col], dx2, rhou, ac, cc, vc, [&](int l, double z, double f) {
+        zt[(long)l * ncol + col] = z;
+        ft[(long)l * ncol + col] = f;
+    });
 }
 // the solve from that table; the next level's values are read before this
 // level's are written
@@ -1913,6 +1922,11 @@ __device__ void thomas_body(const KParams<T> &p, typename V2<T>::t *spec, int TC
         if (sizeof(T) == 8) {
             if (p.th_z) {
                 thomas_column_table(x, p.nz, col, ncol, p.th_z, p.th_f, 1.0 / size2d, p.acoef_d, col == 0);
+            } else if (p.th_eval) {
+                double zl[PPM_MAXZ], fl[PPM_MAXZ];
+                thomas_factors(p.nz, p.hcoef[col], p.dx2, p.rhou_d, p.acoef_d, p.ccoef_d, p.vcoef_d,
+                               [&](int l, double z, double f) { zl[l] = z; fl[l] = f; });
+                thomas_column_table(x, p.nz, 0, 1, zl, fl, 1.0 / size2d, p.acoef_d, col == 0);
             } else {
                 double Floc[PPM_MAXZ];
                 thomas_column<T, double>(p, x, Floc, col, size2d, p.rhou_d, p.acoef_d, p.ccoef_d, p.vcoef_d);

@@ -395,15 +395,15 @@ struct Lin : LinBase {
             tape = nullptr;
             mtape = nullptr;
             tape_steps = 0;
-            if (cudaMalloc(&tape, tape_need * per_step() * sizeof(T)) != cudaSuccess) return GA_ERR_NOMEM;
-            if (nf == 7 && cudaMalloc(&mtape, tape_need * 3 * (size_t)N) != cudaSuccess) return GA_ERR_NOMEM;
+            if (e.take((void **)&tape, tape_need * per_step() * sizeof(T)) != cudaSuccess) return GA_ERR_NOMEM;
+            if (nf == 7 && e.take((void **)&mtape, tape_need * 3 * (size_t)N) != cudaSuccess) return GA_ERR_NOMEM;
             tape_steps = tape_need;
         }
         if (ckpt_need > ckpt_slots) {
             if (ckpt) cudaFree(ckpt);
             ckpt = nullptr;
             ckpt_slots = 0;
-            if (cudaMalloc(&ckpt, ckpt_need * 3 * nf * (size_t)N * sizeof(T)) != cudaSuccess) return GA_ERR_NOMEM;
+            if (e.take((void **)&ckpt, ckpt_need * 3 * nf * (size_t)N * sizeof(T)) != cudaSuccess) return GA_ERR_NOMEM;
             ckpt_slots = ckpt_need;
         }
         return GA_OK;
@@ -435,7 +435,15 @@ struct Lin : LinBase {
             const size_t sb = step_bytes(), cb = 3 * (size_t)nf * N * sizeof(T);
             const size_t have = fr + tape_steps * sb + ckpt_slots * cb;  // the current tape and checkpoints are given back
             const size_t need = (size_t)(nseg + 1) * cb + tot / 10;
-            if (have > need) R = (int)std::min<size_t>((size_t)nseg, (have - need) / ((size_t)K * sb));
+            auto fit = [&](size_t mem) {
+                return mem > need ? (int)std::min<size_t>((size_t)nseg, (mem - need) / ((size_t)K * sb)) : 1;
+            };
+            R = std::max(1, fit(have));
+            // a segment run twice costs more than the tables save
+            if (R < nseg && fit(have + e.table_bytes()) > R) {
+                R = fit(have + e.table_bytes());
+                e.drop_tables();
+            }
         } else {
             cudaGetLastError();
         }

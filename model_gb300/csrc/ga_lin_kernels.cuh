@@ -1352,7 +1352,12 @@ __global__ void k_thomas_adj(KParams<T> p, typename V2<T>::t *spec, int TC)
         if (col == 0 && mean_block) continue;
         if (sizeof(T) == 8 && p.th_z) {
             thomas_T_column_table(x, p.nz, col, ncol, p.th_z, p.th_f, inv_s, p.acoef_d, col == 0);
-        } else if (sizeof(T) == 8 || col == 0) {
+        } else if (sizeof(T) == 8) {
+            double zl[PPM_MAXZ], fl[PPM_MAXZ];
+            thomas_factors(p.nz, p.hcoef[col], p.dx2, p.rhou_d, p.acoef_d, p.ccoef_d, p.vcoef_d,
+                           [&](int l, double z, double f) { zl[l] = z; fl[l] = f; });
+            thomas_T_column_table(x, p.nz, 0, 1, zl, fl, inv_s, p.acoef_d, col == 0);
+        } else if (col == 0) {
             double Floc[PPM_MAXZ];
             thomas_T_column<T2, double>(x, Floc, p.nz, 2.0 * p.hcoef[col] / p.dx2, inv_s, p.rhou_d,
                                         p.acoef_d, p.ccoef_d, p.vcoef_d, col == 0);
