@@ -2050,24 +2050,48 @@ class Engine : public EngineBase {
                 sx_pair = bp;
             }
             // the unfused path (x FFT, Thomas, inverse x FFT) and its level
-            // tile: against the fused kernel where that fits, otherwise
-            // against the current tile, timed once more beside the others
+            // tile: every tile against the fused kernel where that fits,
+            // otherwise the current tile's neighbours against it
             {
                 const int keep_psx = psx, keep_kt = KTx;
                 psx = 0;
-                auto solve = [&] {
-                    float t = 1e30f;
-                    for (int r = 0; r < 3; r++) t = std::min(t, timeit([&] { solve_pressure(1. / 3.); }));
-                    return t;
+                auto solve = [&] { return timeit([&] { solve_pressure(1. / 3.); }); };
+                // Where the scalars' advection runs beside the solve, a tile
+                // that is faster alone may hold up more of that work (FP64
+                // 48x40x32: 2 levels against 8, 60 against 61 us alone, 0.88
+                // against 0.80 ms per two steps), so a tile whose stage takes
+                // longer is out.
+                const bool beside = overlap && !hyd.div && !kp.ice && !cfg.linear_model;
+                auto stage = [&] {
+                    return timeit([&] {
+                        const double st = 1. / 3.;
+                        advect(st, ADV_UV | ADV_WB);
+                        mid_solve = [this, st] {
+                            fork();
+                            OnSide os(this);
+                            advect(st, ADV_TH | (kp.moist ? (ADV_Q | ADV_ZERO) : 0));
+                        };
+                        solve_pressure(st);
+                        join();
+                    });
                 };
-                if (keep_psx == 0) bx = std::min(bx, solve());
-                const int kt = faster_tile(
-                    keep_psx == 0 ? keep_kt : 0, std::min(64, 2 * (NZ - 2)), bx,
-                    [&](int k) { return fft_bytes(kp.ni, k, sizeof(T2)) <= 200 * 1024; },
-                    [&](int k) {
+                auto fits = [&](int k) { return fft_bytes(kp.ni, k, sizeof(T2)) <= 200 * 1024; };
+                int kt;
+                if (keep_psx) {
+                    kt = faster_tile(0, 1, std::min(64, 2 * (NZ - 2)), bx, fits, [&](int k) {
                         set_ktx(k);
                         return solve();
                     });
+                } else {
+                    const float stage_kt = beside ? std::min(stage(), stage()) : 0.f;
+                    bx = std::min(solve(), solve());
+                    kt = faster_tile(keep_kt, std::max(1, keep_kt / 4), std::min(2 * keep_kt, 2 * (NZ - 2)), bx, fits,
+                                     [&](int k) {
+                                         set_ktx(k);
+                                         if (beside && std::min(stage(), stage()) > 1.01f * stage_kt) return 1e30f;
+                                         return std::min(solve(), solve());
+                                     });
+                }
                 set_ktx(kt > 0 ? kt : keep_kt);
                 if (kt <= 0) psx = keep_psx;
                 if (psx == 0) std::snprintf(line, sizeof line, "x level tile %d, ", KTx);
