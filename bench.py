@@ -56,7 +56,7 @@ PASSES_MOIST = {"advect": 22, "div_fft_y": 4, "fft_x": 2, "thomas": 2, "ifft_y_p
 # DRAM bytes per launch (read + write) of the dominant kernel, copied from one
 # ncu capture of the bench command (cold cache) into this table; a run does not
 # measure it.  workload -> (kernel group, kernel, bytes, summary)
-TRAFFIC_NCU = {"thunderstorm": ("advect", "k_advect_march (all fields of a stage)", 65.2e6,
+TRAFFIC_NCU = {"thunderstorm": ("advect", "k_advect_march<2> (all fields of a stage)", 49.7e6,
                                 "profiles/advect_march_thunderstorm_128x128x48_fp32.md")}
 # compulsory bytes per gridpoint-step of an ideally fused step (FP32 moist)
 STEP_BYTES_FP32_MOIST = 540.0

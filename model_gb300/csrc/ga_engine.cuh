@@ -295,7 +295,14 @@ class Engine : public EngineBase {
         }
         {
             cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
-            overlap = c->ny <= nsm;  // kp.nj = NY blocks in the x solve
+            // The scalars' advection beside the solve pays where the solve's
+            // launches leave SMs idle.  ms per four steps of NZ = 48 off / on:
+            // FP32 96x96 0.837 / 0.800, 64x256 1.170 / 1.175, 128x128 1.210 /
+            // 1.230, 160x160 1.676 / 1.686, 256x256 3.74 / 3.90; FP64 96x96
+            // 10.25 / 9.86, 128x128 16.85 / 16.51, 256x256 65.3 / 63.0.  The line
+            // dates from an x solve of NY blocks (it has NY/2 + 1 in FP32 and
+            // tiles over every SM in FP64): near break-even where it lies in FP32
+            overlap = c->ny <= nsm;
             if (const char *ev = std::getenv("GA_OVERLAP")) overlap_rec = overlap = std::strcmp(ev, "0") != 0;
         }
         const bool moist = c->microphysics_option >= 1;

@@ -21,12 +21,14 @@
 // fetched once, both faces' arithmetic runs on packed pairs of levels
 // (fma.rn.f32x2, half the instructions of scalar code), and fields run as
 // separate blocks, which gives a small grid enough of them.  Bound: latency
-// and instruction fetch (128x128x48: issue 43% active, DRAM and L1 below 40%,
-// stalls on loads 3.4 and on instruction fetch 2.3 cycles an issue), so small
-// grids run two blocks of 126 registers an SM (64x64x40 17 against 20 us a
-// stage at three blocks of 80), large ones three (512x512x64 820 against
-// 870).  All fields of a stage, against k_advect_quad's best tile: 64x64x40
-// 21.5 -> 14.9 us, 128x128x48 67 -> 47 us, 512x512x64 1022 -> 820 us.
+// (all fields of a stage at 128x128x48, 49.6 us cold: issue 39% active, L1 51%,
+// stalls an issue on loads 3.5, fixed latency 1.6, barriers 1.0).  Small grids
+// run two blocks of 128 registers an SM (64x64x40 17 against 20 us a stage at
+// three blocks of 80), large ones three, although at 80 registers a thread
+// spills 304 bytes of stores and 184 of loads (512x512x64 820 against 870 us;
+// 814 cold: issue 47%, L1 66%, stalls on loads 6.0).  All fields of a stage,
+// against k_advect_quad's best tile: 64x64x40 21.5 -> 14.9 us, 128x128x48 67 ->
+// 47 us, 512x512x64 1022 -> 820 us.
 //
 // Per level the arithmetic is that of the k_advect_tile face and tendency
 // functions, expression for expression.
@@ -161,8 +163,8 @@ struct MarchGeom {
 };
 // TJ: as many thread rows as fit AM_THREADS, the tiles of a row of equal size.
 // LI: a chunk starts with six planes to fetch and one extra east face, so it
-// is as long as leaves about two waves of three blocks on each SM, at least 4
-// and at most 16 columns: 64x64x40 took 15 us a stage with 4 and 24 with 8,
+// is as long as leaves about six blocks for each SM (three waves of two blocks
+// or two of three), at least 4 and at most 16 columns: 64x64x40 took 15 us a stage with 4 and 24 with 8,
 // 128x128x48 49 with 5 and 64 with 16 (all fields, one stream); at 512x512x64
 // 16 and 32 are equal.  li > 0 fixes it.
 __host__ inline MarchGeom march_geom(int nx, int ny, int nz, int njobs, int nsm, int li = 0)
