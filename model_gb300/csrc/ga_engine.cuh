@@ -1887,7 +1887,8 @@ class Engine : public EngineBase {
     {
         cudaSetDevice(device);
         refresh_base();
-        const int nsnap = nprog + 2;
+        T *wcur = hyd.div ? buf[FW][ci[FW]] : nullptr;  // the hydrostatic set's w lives in its current slot
+        const int nsnap = nprog + 2 + (wcur ? 1 : 0);
         T *snap = nullptr;
         if (take((void **)&snap, (size_t)nsnap * N * sizeof(T)) != cudaSuccess) return GA_ERR_NOMEM;
         refresh_base();  // (with the faces given back)
@@ -1895,6 +1896,7 @@ class Engine : public EngineBase {
             cudaMemcpyAsync(snap + (size_t)f * N, buf[f][pi_[f]], N * sizeof(T), cudaMemcpyDeviceToDevice, stream);
         cudaMemcpyAsync(snap + (size_t)nprog * N, pi, N * sizeof(T), cudaMemcpyDeviceToDevice, stream);
         cudaMemcpyAsync(snap + (size_t)(nprog + 1) * N, vt, N * sizeof(T), cudaMemcpyDeviceToDevice, stream);
+        if (wcur) cudaMemcpyAsync(snap + (size_t)(nprog + 2) * N, wcur, N * sizeof(T), cudaMemcpyDeviceToDevice, stream);
         cudaEvent_t ea, eb;
         cudaEventCreate(&ea);
         cudaEventCreate(&eb);
@@ -2113,6 +2115,7 @@ class Engine : public EngineBase {
             cudaMemcpyAsync(buf[f][pi_[f]], snap + (size_t)f * N, N * sizeof(T), cudaMemcpyDeviceToDevice, stream);
         cudaMemcpyAsync(pi, snap + (size_t)nprog * N, N * sizeof(T), cudaMemcpyDeviceToDevice, stream);
         cudaMemcpyAsync(vt, snap + (size_t)(nprog + 1) * N, N * sizeof(T), cudaMemcpyDeviceToDevice, stream);
+        if (wcur) cudaMemcpyAsync(wcur, snap + (size_t)(nprog + 2) * N, N * sizeof(T), cudaMemcpyDeviceToDevice, stream);
         const int rc = sync_status();
         cudaEventDestroy(ea);
         cudaEventDestroy(eb);
